@@ -1,0 +1,524 @@
+"""The work whose speed this framework is judged by: single layers and blocks of the decoders it serves, and one whole
+decode step, each through the entry point that a model calls.
+
+Sizes are those of Llama-3-8B (hidden 4096, 32 query heads over 8 key/value heads of 128, feed-forward 14336, vocabulary
+128256) and of the w2048 configuration of the other designs (hidden 2048, 16 heads).  Sequences of a batch differ in length:
+each holds between half of the stated number of tokens and all of it.  Steps of single tokens run as captured graphs where
+the serving engine replays them (whole step, layers of the other designs); single operators are called one by one."""
+import math
+import random
+
+import torch
+
+from scalellm_b200.decode_step import BlockPool, GraphedStep, LlamaArgs, LlamaDecoder, StepBuffers, build_step_batch
+from scalellm_b200.layers import (B200AttnHandler, ColumnParallelLinear, ColumnParallelQLinear, GatedDeltaMixer, KVCache,
+                                  LatentAttention, LatentKVCache, QuantArgs, SinkAttention, SparseMoE, SumNormResidual)
+from scalellm_b200.model_parallel import ParallelArgs
+
+BF16 = torch.bfloat16
+EPS = 1e-5
+HIDDEN, HEADS, KV_HEADS, HEAD, FF, VOCAB = 4096, 32, 8, 128, 14336, 128256          # Llama-3-8B
+WIDTH, ROT, RANK, EXPERTS, TOP, EXPERT_FF, TAPS, LOW = 2048, 64, 512, 8, 2, 1408, 4, 32
+PROJECTIONS = [(HIDDEN, HIDDEN + 2 * KV_HEADS * HEAD), (HIDDEN, HIDDEN), (HIDDEN, 2 * FF), (FF, HIDDEN)]   # in, out
+
+
+def listed():
+    return [
+        # one user's decoded token through an int4 projection: the smallest call there is
+        dict(name="int4_one_row", kind="int4", rows=1, k=HIDDEN, n=HIDDEN, quant="awq", group=128),
+        # the same for a full decode batch, the widest projection: the framework's headline workload
+        dict(name="int4_batch", kind="int4", rows=64, k=HIDDEN, n=2 * FF, quant="awq", group=128),
+        # a prompt of odd length through the deepest int4 projection
+        dict(name="int4_prompt", kind="int4", rows=1027, k=FF, n=HIDDEN, quant="gptq", group=128),
+        # the vocabulary projection of a decode batch: bf16 in every configuration
+        dict(name="bf16_head", kind="bf16", rows=64, k=HIDDEN, n=VOCAB),
+        # a prompt portion through an unquantised projection
+        dict(name="bf16_prompt", kind="bf16", rows=1999, k=HIDDEN, n=2 * FF),
+        # decoding over a paged cache at the headline batch and context
+        dict(name="attention_decode", kind="attention", seqs=64, new=1, cached=2047, block=8),
+        # chunked prefill: portions of prompts over what earlier portions left in the cache
+        dict(name="attention_prompt", kind="attention", seqs=8, new=512, cached=1536, block=8),
+        # a whole decode step with logits (int4 layers, bf16 vocabulary projection), metadata uploaded, graph replayed
+        dict(name="llama_step", kind="step", seqs=16, cached=1023, layers=4, block=8),
+        # attention over compressed latents, prompts
+        dict(name="latent_prompt", kind="latent", seqs=4, new=2048, cached=0, heads=16, window=0),
+        # attention with a distance bias and a sink, prompts, with the residual and norm that follow it
+        dict(name="sink_prompt", kind="sink", seqs=4, new=2048, cached=0, heads=16),
+        # the gated delta rule over prompts
+        dict(name="delta_prompt", kind="delta", seqs=8, new=1024, heads=16),
+        # routed experts of a decode batch
+        dict(name="experts_decode", kind="experts", rows=16),
+    ]
+
+
+def draw(rng):
+    """Another case of the same ranges; none does more work than the largest listed one of its kind."""
+    log = lambda lo, hi: int(round(math.exp(rng.uniform(math.log(lo), math.log(hi + 0.49)))))
+    kind = rng.choice(["int4", "int4", "bf16", "bf16", "attention", "attention", "step", "latent", "sink", "delta",
+                       "experts"])
+    if kind == "int4":
+        k, n = rng.choice(PROJECTIONS)
+        return dict(kind=kind, rows=log(1, 1027), k=k, n=n, quant=rng.choice(["awq", "gptq"]), group=rng.choice([64, 128]))
+    if kind == "bf16":
+        k, n = rng.choice(PROJECTIONS + [(HIDDEN, VOCAB)])
+        return dict(kind=kind, rows=log(1, 64 if n == VOCAB else 1999), k=k, n=n)
+    if kind == "step":
+        return dict(kind=kind, seqs=log(1, 64), cached=log(64, 1023), layers=4, block=rng.choice([8, 16]))
+    if kind == "delta":
+        new = log(2, 1024)
+        return dict(kind=kind, seqs=log(1, max(1, min(64, 8192 // new))), new=new, heads=rng.choice([16, 32]) if new <= 512 else 16)
+    if kind == "experts":
+        return dict(kind=kind, rows=log(1, 2048))
+    heads = rng.choice([16, 32])
+    new = rng.choice([1, log(2, 2048)])
+    cached = log(16, 4095) if new == 1 else rng.choice([0, log(16, 2048)])
+    # (query, key) pairs of all heads: at most what four prompts of 2048 tokens and 16 heads have
+    seqs = log(1, max(1, min(64, (64 * 1024 if new > 1 else 1 << 18) // (new + cached), 4 * 2048 // new)))
+    while seqs > 1 and seqs * heads * new * (cached + new / 2) > 4 * 16 * 2048 * 1024:
+        seqs -= 1
+    if seqs * heads * new * (cached + new / 2) > 4 * 16 * 2048 * 1024:
+        cached, heads = 0, 16
+    if kind == "attention":
+        return dict(kind=kind, seqs=seqs, new=min(new, 512), cached=cached, block=rng.choice([8, 16]))
+    if kind == "latent":
+        return dict(kind=kind, seqs=seqs, new=new, cached=cached, heads=heads, window=rng.choice([0, 512]))
+    return dict(kind=kind, seqs=seqs, new=new, cached=cached, heads=heads)
+
+
+# ------------------------------------------------------------------------------------------------------------ inputs
+def _lengths(case):
+    """(new tokens, cached tokens) of every sequence; the first has the stated numbers."""
+    r = random.Random("%d %d %d" % (case["seqs"], case.get("new", 1), case.get("cached", 0)))
+    part = lambda n, first: n if first or n <= 1 else r.randint((n + 1) // 2, n)
+    return [(part(case.get("new", 1), i == 0), part(case.get("cached", 0), i == 0)) for i in range(case["seqs"])]
+
+
+def _generator(seed):
+    return torch.Generator(device="cuda").manual_seed(seed)
+
+
+def _normal(g, *shape, std=1.0, mean=0.0, dtype=BF16):
+    return (torch.randn(shape, generator=g, device="cuda") * std + mean).to(dtype)
+
+
+def _weight(g, n_out, n_in):
+    return _normal(g, n_out, n_in, std=n_in ** -0.5)
+
+
+def _words(g, *shape):
+    return torch.randint(-2 ** 31, 2 ** 31, shape, generator=g, device="cuda", dtype=torch.int64).to(torch.int32)
+
+
+def _int4_weights(g, k, n, quant, group):
+    """A checkpoint's tensors: uniform 4-bit values (and zero points), positive scales per group; rows keep their size."""
+    scales = ((torch.randn((k // group, n), generator=g, device="cuda").abs() + 0.1) * 0.15 * k ** -0.5).to(BF16)
+    if quant == "awq":
+        return dict(qweight=_words(g, k, n // 8), qzeros=_words(g, k // group, n // 8), scales=scales)
+    return dict(qweight=_words(g, k // 8, n), qzeros=None, scales=scales)
+
+
+def _batch(case, seed):
+    """The step's host metadata and cache size: blocks of every sequence scattered over the pool."""
+    lens, bs = _lengths(case), case.get("block", 16)
+    n_blocks = sum(-(-(a + b) // bs) for a, b in lens) + 8
+    pool = BlockPool(n_blocks, bs, seed=seed)
+    seqs = [pool.open_sequence() for _ in lens]
+    for s, (a, b) in zip(seqs, lens):
+        pool.reserve(s, a + b)
+    r = random.Random(seed)
+    hb = build_step_batch(pool, seqs, [[r.randrange(32000) for _ in range(a)] for a, _ in lens], [b for _, b in lens],
+                          list(range(len(lens))))
+    return hb, n_blocks, bs
+
+
+def _buffers(hb, n_blocks):
+    return StepBuffers(torch.device("cuda"), len(hb.tokens), len(hb.q_cu_lens) - 1, n_blocks)
+
+
+def _slots(case, seed):
+    """Cache slots of every sequence's tokens in order, from the block table as the metadata carries it."""
+    hb, _, bs = _batch(case, seed)
+    out = []
+    for i, (a, b) in enumerate(_lengths(case)):
+        table = torch.from_numpy(hb.block_tables[hb.cu_block_lens[i]: hb.cu_block_lens[i + 1]].astype("int64"))
+        out.append((table[:, None] + torch.arange(bs)).reshape(-1)[: a + b].cuda())
+    return out
+
+
+def _inputs(case, seed):
+    """Every tensor of the case, from the seed alone: what prepare() loads and exact() computes with."""
+    g, kind = _generator(seed), case["kind"]
+    if kind == "int4":
+        return dict(x=_normal(g, case["rows"], case["k"]),
+                    w=_int4_weights(g, case["k"], case["n"], case["quant"], case["group"]))
+    if kind == "bf16":
+        return dict(x=_normal(g, case["rows"], case["k"]), w=_normal(g, case["n"], case["k"], std=0.02))
+    if kind == "experts":
+        ff = EXPERT_FF
+        return dict(h=_normal(g, case["rows"], WIDTH), router=_weight(g, EXPERTS, WIDTH),
+                    gate=_normal(g, EXPERTS, ff, WIDTH, std=WIDTH ** -0.5),
+                    up=_normal(g, EXPERTS, ff, WIDTH, std=WIDTH ** -0.5),
+                    down=_normal(g, EXPERTS, WIDTH, ff, std=ff ** -0.5))
+    rows = sum(a for a, _ in _lengths(case))
+    if kind == "delta":
+        H, G, d = case["heads"], case["heads"] // 2, HEAD
+        u = lambda *shape: torch.rand(shape, generator=g, device="cuda")
+        return dict(h=_normal(g, rows, WIDTH), w={
+            "q": _weight(g, G * d, WIDTH), "k": _weight(g, G * d, WIDTH), "v": _weight(g, H * d, WIDTH),
+            "q.conv": _weight(g, G * d, TAPS), "k.conv": _weight(g, G * d, TAPS), "v.conv": _weight(g, H * d, TAPS),
+            "b": _weight(g, H, WIDTH), "a1": _weight(g, LOW, WIDTH), "a2": _weight(g, H * d, LOW),
+            "g1": _weight(g, LOW, WIDTH), "g2": _weight(g, H * d, LOW), "o": _weight(g, WIDTH, H * d),
+            "A_log": torch.log(0.5 + 4.0 * u(H)).to(BF16), "dt_bias": (-4.0 + 3.0 * u(H * d)).to(BF16),
+            "norm": _normal(g, d, std=0.2, mean=1.0)})
+    n_slots = _batch(case, seed)[1] * case.get("block", 16)
+    if kind == "attention":
+        return dict(q=_normal(g, rows, HEADS, HEAD), k=_normal(g, n_slots, KV_HEADS, HEAD),
+                    v=_normal(g, n_slots, KV_HEADS, HEAD))
+    if kind == "step":
+        layer = lambda: dict(
+            qkv=_int4_weights(g, HIDDEN, (HEADS + 2 * KV_HEADS) * HEAD, "awq", 128),
+            o=_int4_weights(g, HIDDEN, HIDDEN, "awq", 128), gate_up=_int4_weights(g, HIDDEN, 2 * FF, "awq", 128),
+            down=_int4_weights(g, FF, HIDDEN, "awq", 128), input_norm=_normal(g, HIDDEN, std=0.2, mean=1.0),
+            post_norm=_normal(g, HIDDEN, std=0.2, mean=1.0), k=_normal(g, n_slots, KV_HEADS, HEAD),
+            v=_normal(g, n_slots, KV_HEADS, HEAD))
+        return dict(layers=[layer() for _ in range(case["layers"])], embed=_normal(g, VOCAB, HIDDEN, std=0.02),
+                    norm=_normal(g, HIDDEN, std=0.2, mean=1.0), head=_normal(g, VOCAB, HIDDEN, std=0.02))
+    H = case["heads"]
+    if kind == "latent":
+        cache = torch.randn((n_slots, RANK + ROT), generator=g, device="cuda").to(BF16)
+        return dict(h=_normal(g, rows, WIDTH), cache=cache, w={
+            "q": _weight(g, H * (HEAD + ROT), WIDTH), "dkv": _weight(g, RANK + ROT, WIDTH),
+            "dkv.norm": _normal(g, RANK, std=0.2, mean=1.0), "uk": _weight(g, H * HEAD, RANK),
+            "uv": _weight(g, H * HEAD, RANK), "o": _weight(g, WIDTH, H * HEAD)})
+    G = H // 4
+    u = lambda: (0.05 + 0.5 * torch.rand((H,), generator=g, device="cuda")).to(BF16)
+    return dict(h=_normal(g, rows, WIDTH), x=_normal(g, rows, WIDTH, dtype=torch.float32),
+                k=_normal(g, n_slots, G, HEAD), v=_normal(g, n_slots, G, HEAD), norm=_normal(g, WIDTH, std=0.2, mean=1.0), w={
+                    "q": _weight(g, H * HEAD, WIDTH), "k": _weight(g, G * HEAD, WIDTH), "v": _weight(g, G * HEAD, WIDTH),
+                    "o": _weight(g, WIDTH, H * HEAD), "r1": u(), "r2": u(), "sink": _normal(g, H)})
+
+
+# ----------------------------------------------------------------------------------------------------------- the calls
+class _Replay:
+    """A step as the serving engine keeps it: run twice, then captured and replayed."""
+
+    def __init__(self, fn):
+        s = torch.cuda.Stream()
+        s.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(s):
+            fn()
+            fn()
+        torch.cuda.current_stream().wait_stream(s)
+        torch.cuda.synchronize()
+        self.graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(self.graph):
+            self.out = fn()
+
+    def __call__(self):
+        self.graph.replay()
+        return self.out
+
+
+def _inv_freq():
+    return 10000.0 ** (-torch.arange(0, ROT, 2, dtype=torch.float64) / ROT)
+
+
+def prepare(case, seed):
+    dev, alone, t = torch.device("cuda"), ParallelArgs(0, 1, None), _inputs(case, seed)
+    kind = case["kind"]
+    if kind == "int4":
+        qa = QuantArgs(case["quant"], 4, case["group"], False, case["quant"] == "gptq", case["quant"] == "awq")
+        layer = ColumnParallelQLinear(case["k"], case["n"], False, False, qa, alone, dev)
+        layer.load_state_dict(t["w"])
+        layer(t["x"][:1])                      # loading ends with packed weights
+        return lambda: layer(t["x"])
+    if kind == "bf16":
+        layer = ColumnParallelLinear(case["k"], case["n"], False, alone, BF16, dev)
+        layer.load_state_dict({"weight": t["w"]})
+        return lambda: layer(t["x"])
+    if kind == "experts":
+        layer = SparseMoE(t["router"], t["gate"], t["up"], t["down"], TOP, "silu")
+        step = lambda: layer(t["h"])
+        return _Replay(step) if case["rows"] <= 64 else step
+    if kind == "step":
+        hb, n_blocks, bs = _batch(case, seed)
+        args = LlamaArgs(n_layers=case["layers"])
+        model = LlamaDecoder(args, QuantArgs("awq", 4, 128), alone, dev)
+        for i, layer in enumerate(t["layers"]):
+            model.load_layer(i, layer)
+        model.embed.copy_(t["embed"])
+        model.lm_head.weight.copy_(t["head"])
+        model.final_norm.weight.copy_(t["norm"])
+        model.alloc_kv(n_blocks, bs, randomize=False)
+        for cache, layer in zip(model.kv_caches, t["layers"]):
+            cache.key_cache.copy_(layer["k"])
+            cache.value_cache.copy_(layer["v"])
+        bufs = _buffers(hb, n_blocks)
+        step = GraphedStep(model, bufs, hb, greedy=False)
+        caches = [c for kv in model.kv_caches for c in kv.get_kv_cache()]
+
+        def whole():
+            bufs.upload(hb)
+            return [step.replay()] + caches
+        return whole
+    if kind == "delta":
+        n_seq = case["seqs"]
+        hb, n_blocks, _ = _batch(case, seed)
+        _, pos, prm = _buffers(hb, n_blocks).upload(hb)
+        layer = GatedDeltaMixer(t["w"], case["heads"], case["heads"] // 2, HEAD, HEAD, 1e-6, EPS, n_seq, BF16, dev)
+        return lambda: [layer(t["h"], pos, prm), layer.state, layer.filter_state]
+    hb, n_blocks, bs = _batch(case, seed)
+    _, pos, prm = _buffers(hb, n_blocks).upload(hb)
+    if kind == "attention":
+        handler, cache = B200AttnHandler(HEAD ** -0.5), KVCache(n_blocks, bs, KV_HEADS, HEAD, BF16, dev)
+        cache.key_cache.copy_(t["k"])
+        cache.value_cache.copy_(t["v"])
+
+        def attend():
+            out = torch.empty_like(t["q"])
+            handler.batch_decode(t["q"], cache, prm, -1, out)
+            return out
+        return attend
+    if kind == "latent":
+        layer = LatentAttention(t["w"], case["heads"], HEAD, ROT, HEAD, RANK, (HEAD + ROT) ** -0.5, _inv_freq(), 1.0, ROT,
+                                EPS, BF16, dev, window=case["window"])
+        cache = LatentKVCache(n_blocks, bs, RANK, ROT, BF16, dev)
+        cache.rows.copy_(t["cache"])
+        step = lambda: [layer(t["h"], pos, cache, prm), cache.rows]
+    else:
+        H = case["heads"]
+        layer = SinkAttention(t["w"], H, H // 4, HEAD, HEAD, HEAD ** -0.5, 0.1, 1024, None, EPS, BF16, dev)
+        norm = SumNormResidual(t["norm"], 1.0, EPS)
+        cache = KVCache(n_blocks, bs, H // 4, HEAD, BF16, dev)
+        cache.key_cache.copy_(t["k"])
+        cache.value_cache.copy_(t["v"])
+        x_out = torch.empty_like(t["x"])
+
+        def step():
+            y, _ = layer(t["h"], pos, cache, prm)
+            x, h = norm(t["x"], y, BF16, x_out)
+            return [x, h, cache.key_cache, cache.value_cache]
+    return _Replay(step) if case["new"] == 1 else step
+
+
+def run(state):
+    return state()
+
+
+# ------------------------------------------------------------------------------------------------------ what it takes
+def work(case):
+    kind = case["kind"]
+    if kind in ("int4", "bf16"):
+        m, k, n = case["rows"], case["k"], case["n"]
+        w = k * n * 2 if kind == "bf16" else k * n // 2 + (k // case["group"]) * n * (2 + (0.5 if case["quant"] == "awq" else 0))
+        return {"bytes": w + 2 * m * (k + n), "flops": 2 * m * k * n}
+    if kind == "experts":
+        m, one = case["rows"], 3 * WIDTH * EXPERT_FF
+        used = EXPERTS * (1 - (1 - TOP / EXPERTS) ** m)            # experts that some row chooses
+        return {"bytes": used * one * 2 + 4 * m * WIDTH, "flops": 2 * m * TOP * one}
+    lens = _lengths(case)
+    rows, seen = sum(a for a, _ in lens), sum(a + b for a, b in lens)
+    pairs = lambda w: sum(sum(min(b + i + 1, w) for i in range(a)) for a, b in lens)
+    full = pairs(1 << 40)
+    if kind == "attention":
+        return {"bytes": 4 * seen * KV_HEADS * HEAD + 4 * rows * HEADS * HEAD, "flops": 4 * full * HEADS * HEAD}
+    if kind == "step":
+        n_w = case["layers"] * sum(k * n for k, n in PROJECTIONS)
+        kv = 4 * (seen + rows) * KV_HEADS * HEAD * case["layers"]
+        return {"bytes": n_w * (0.5 + 2.5 / 128) + VOCAB * HIDDEN * 2 + kv + 2 * rows * (VOCAB + HIDDEN),
+                "flops": 2 * rows * (n_w + VOCAB * HIDDEN) + 4 * full * case["layers"] * HEADS * HEAD}
+    H, d = case["heads"], HEAD
+    if kind == "delta":
+        proj = WIDTH * (3 * H * d + H + 2 * LOW) + 2 * LOW * H * d                  # q and k have half the heads
+        return {"bytes": 2 * proj + 4 * rows * WIDTH + 4 * case["seqs"] * (H * d * d + (TAPS - 1) * 2 * H * d),
+                "flops": 2 * rows * proj + 7 * rows * H * d * d}
+    if kind == "latent":
+        seen_pairs = pairs(case["window"] or 1 << 40)
+        proj = WIDTH * (H * (d + ROT) + RANK + ROT + H * d)
+        folded = 2 * rows * H * RANK * 2 * d + 2 * seen_pairs * H * (2 * RANK + ROT)           # queries meet the latents
+        plain = 2 * seen * H * RANK * 2 * d + 2 * seen_pairs * H * (2 * d + ROT)              # keys and values made first
+        return {"bytes": 2 * (proj + 2 * H * d * RANK) + 2 * (seen + rows) * (RANK + ROT) + 4 * rows * WIDTH,
+                "flops": 2 * rows * proj + min(folded, plain)}
+    G = H // 4
+    proj = WIDTH * (2 * H + 2 * G) * d
+    return {"bytes": 2 * proj + 4 * (seen + rows) * G * d + rows * WIDTH * (2 + 4 + 4 + 2),
+            "flops": 2 * rows * proj + 4 * full * H * d}
+
+
+def tolerance(case):
+    """About four times the error measured against exact(): bf16 results and bf16 rows between the products of a block."""
+    return {"int4": {"rel": 0.01}, "bf16": {"rel": 0.007}, "attention": {"rel": 0.01}, "step": {"rel": 0.07},
+            "latent": {"rel": 0.02}, "sink": {"rel": 0.01}, "delta": {"rel": 0.014}, "experts": {"rel": 0.02}}[case["kind"]]
+
+
+# ---------------------------------------------------------------------------------------------------- in 64-bit numbers
+def _unpack(words, dim, order):
+    """Eight 4-bit values of every word, along `dim`; value j sits in nibble order[j]."""
+    v = torch.stack([(words.to(torch.int64) >> (4 * s)) & 15 for s in order], dim=dim + 1)
+    return v.reshape([n * (8 if i == dim else 1) for i, n in enumerate(words.shape)])
+
+
+def _int4_exact(w, quant, group):
+    """[k, n] in 64 bits."""
+    if quant == "awq":
+        order = [0, 4, 1, 5, 2, 6, 3, 7]
+        q, z = _unpack(w["qweight"], 1, order), _unpack(w["qzeros"], 1, order).repeat_interleave(group, dim=0)
+    else:
+        q, z = _unpack(w["qweight"], 0, range(8)), 8
+    return (q - z).double() * w["scales"].double().repeat_interleave(group, dim=0)
+
+
+def _rms(x, w=1.0):
+    return x / torch.sqrt((x * x).mean(dim=-1, keepdim=True) + EPS) * w
+
+
+def _visible(pos, n, window=0):
+    j = torch.arange(n, device="cuda")
+    ok = j[None, :] <= pos[:, None]
+    return ok & (pos[:, None] - j[None, :] < window) if window else ok
+
+
+def _attend(q, k, v, pos, scale, bias=None, sink=None, window=0):
+    """q [T, H, d] over k, v [n, G, d]: H / G query heads per key head; bias(h) [T, n] is added to the scores."""
+    out = torch.empty(q.shape[0], q.shape[1], v.shape[2], dtype=torch.float64, device="cuda")
+    per = q.shape[1] // k.shape[1]
+    ok = _visible(pos, k.shape[0], window)
+    for h in range(q.shape[1]):
+        s = (q[:, h] @ k[:, h // per].T) * scale
+        if bias is not None:
+            s = s + bias(h)
+        s = s.masked_fill(~ok, -math.inf)
+        if sink is not None:
+            s = torch.cat([s, sink[h].expand(s.shape[0], 1)], dim=1)
+        out[:, h] = torch.softmax(s, dim=-1)[:, : k.shape[0]] @ v[:, h // per]
+    return out
+
+
+def _turn(x, pos, f, half):
+    """Rotary turn of x [T, ..., 2 len(f)]: neighbours, or channel t with t + len(f)."""
+    a = (pos.double()[:, None] * f.cuda()[None, :]).reshape([x.shape[0]] + [1] * (x.dim() - 2) + [f.numel()])
+    c, s = torch.cos(a), torch.sin(a)
+    if half:
+        u, v = x[..., : f.numel()], x[..., f.numel():]
+        return torch.cat([u * c - v * s, v * c + u * s], dim=-1)
+    u, v = x[..., 0::2], x[..., 1::2]
+    return torch.stack([u * c - v * s, v * c + u * s], dim=-1).flatten(-2)
+
+
+def _llama_frequencies():
+    f = 500000.0 ** (-torch.arange(0, HEAD, 2, dtype=torch.float64) / HEAD)
+    length, smooth = 2 * math.pi / f, (8192 / (2 * math.pi / f) - 1.0) / 3.0
+    mid = (1 - smooth) * f / 8.0 + smooth * f
+    return torch.where(length < 8192 / 4.0, f, torch.where(length > 8192 / 1.0, f / 8.0, mid))
+
+
+def exact(case, seed):
+    t, kind = _inputs(case, seed), case["kind"]
+    D = lambda x: x.double()
+    silu = torch.nn.functional.silu
+    if kind == "int4":
+        return D(t["x"]) @ _int4_exact(t["w"], case["quant"], case["group"])
+    if kind == "bf16":
+        return torch.cat([D(t["x"]) @ D(w).T for w in t["w"].split(16384)], dim=1)
+    if kind == "experts":
+        h = D(t["h"])
+        s, ids = torch.sigmoid(h @ D(t["router"]).T).topk(TOP, dim=-1)
+        out = torch.zeros_like(h)
+        for e in range(EXPERTS):
+            row, j = (ids == e).nonzero(as_tuple=True)
+            x = h[row] * s[row, j][:, None]
+            out.index_add_(0, row, (silu(x @ D(t["gate"][e]).T) * (x @ D(t["up"][e]).T)) @ D(t["down"][e]).T)
+        return out
+    lens = _lengths(case)
+    starts = [sum(a for a, _ in lens[:i]) for i in range(len(lens))]
+    where = lambda i: (slice(starts[i], starts[i] + lens[i][0]), torch.arange(lens[i][1], sum(lens[i]), device="cuda"))
+    if kind == "delta":
+        return _delta_exact(case, t, starts, lens)
+    slots = _slots(case, seed)
+    if kind == "attention":
+        out = torch.empty(t["q"].shape, dtype=torch.float64, device="cuda")
+        for i, sl in enumerate(slots):
+            rows, pos = where(i)
+            out[rows] = _attend(D(t["q"][rows]), D(t["k"][sl]), D(t["v"][sl]), pos, HEAD ** -0.5)
+        return out
+    if kind == "step":
+        hb, _, _ = _batch(case, seed)
+        f, pos_all = _llama_frequencies(), torch.from_numpy(hb.positions).cuda()
+        h = D(t["embed"][torch.from_numpy(hb.tokens).cuda().long()])
+        caches = []
+        for layer in t["layers"]:
+            W = lambda name: _int4_exact(layer[name], "awq", 128)
+            q, k, v = (_rms(h, D(layer["input_norm"])) @ W("qkv")).reshape(len(h), -1, HEAD).split([HEADS, KV_HEADS, KV_HEADS], 1)
+            q, k = _turn(q, pos_all, f, True), _turn(k, pos_all, f, True)
+            K, V, o = D(layer["k"]), D(layer["v"]), torch.empty_like(q)
+            for i, sl in enumerate(slots):
+                rows, pos = where(i)
+                K[sl[pos]], V[sl[pos]] = k[rows], v[rows]
+                o[rows] = _attend(q[rows], K[sl], V[sl], pos, HEAD ** -0.5)
+            h = h + o.reshape(len(h), -1) @ W("o")
+            gate, up = (_rms(h, D(layer["post_norm"])) @ W("gate_up")).chunk(2, dim=1)
+            h = h + (silu(gate) * up) @ W("down")
+            caches += [K, V]
+        h = _rms(h, D(t["norm"]))
+        return [torch.cat([h @ D(w).T for w in t["head"].split(16384)], dim=1)] + caches
+    w, h, H = {n: D(x) for n, x in t["w"].items()}, D(t["h"]), case["heads"]
+    if kind == "latent":
+        rows_cache, f, o = D(t["cache"]), _inv_freq(), torch.empty(len(h), H * HEAD, dtype=torch.float64, device="cuda")
+        uk, uv = w["uk"].reshape(H, HEAD, RANK), w["uv"].reshape(H, HEAD, RANK)
+        for i, sl in enumerate(slots):
+            rows, pos = where(i)
+            q = (h[rows] @ w["q"].T).reshape(len(pos), H, HEAD + ROT)
+            d = h[rows] @ w["dkv"].T
+            rows_cache[sl[pos]] = torch.cat([_rms(d[:, :RANK], w["dkv.norm"]), _turn(d[:, RANK:], pos, f, False)], dim=-1)
+            c, kr, ok = rows_cache[sl][:, :RANK], rows_cache[sl][:, RANK:], _visible(pos, len(sl), case["window"])
+            qr = _turn(q[..., HEAD:], pos, f, False)
+            for j in range(H):
+                s = ((q[:, j, :HEAD] @ uk[j]) @ c.T + qr[:, j] @ kr.T) * (HEAD + ROT) ** -0.5
+                o[rows, j * HEAD: (j + 1) * HEAD] = (torch.softmax(s.masked_fill(~ok, -math.inf), dim=-1) @ c) @ uv[j].T
+        return [o @ w["o"].T, rows_cache]
+    G = H // 4
+    K, V, o = D(t["k"]), D(t["v"]), torch.empty(len(h), H * HEAD, dtype=torch.float64, device="cuda")
+    for i, sl in enumerate(slots):
+        rows, pos = where(i)
+        q = _rms((h[rows] @ w["q"].T).reshape(len(pos), H, HEAD))
+        q = q * (1.0 + 0.1 * torch.log(torch.floor((pos.double() + 1) / 1024) + 1.0))[:, None, None]
+        K[sl[pos]] = _rms((h[rows] @ w["k"].T).reshape(len(pos), G, HEAD))
+        V[sl[pos]] = (h[rows] @ w["v"].T).reshape(len(pos), G, HEAD)
+        far = (pos[:, None] - torch.arange(len(sl), device="cuda")[None, :]).clamp(min=0).double()
+        bias = lambda j: -w["r1"][j] * torch.log(1.0 + w["r2"][j] * far)
+        o[rows] = _attend(q, K[sl], V[sl], pos, HEAD ** -0.5, bias, w["sink"]).reshape(len(pos), -1)
+    x = _rms(D(t["x"]) + o @ w["o"].T, D(t["norm"]))
+    return [x, x, K, V]
+
+
+def _delta_exact(case, t, starts, lens):
+    w, h, H, d = {n: x.double() for n, x in t["w"].items()}, t["h"].double(), case["heads"], HEAD
+    G, n_seq, T = H // 2, len(lens), max(a for a, _ in lens)
+    silu = torch.nn.functional.silu
+    padded = torch.zeros(n_seq, T, WIDTH, dtype=torch.float64, device="cuda")
+    for i, (a, _) in enumerate(lens):
+        padded[i, :a] = h[starts[i]: starts[i] + a]
+    raw = torch.cat([padded @ w[n].T for n in ("q", "k", "v")], dim=-1)
+    filt = torch.cat([w[n + ".conv"] for n in ("q", "k", "v")])
+    before = torch.cat([torch.zeros_like(raw[:, : TAPS - 1]), raw], dim=1)
+    y = silu(sum(before[:, i: i + T] * filt[:, i] for i in range(TAPS)))
+    q, k, v = y.split([G * d, G * d, H * d], dim=-1)
+    unit = lambda z: (z / torch.sqrt((z * z).sum(dim=-1, keepdim=True) + 1e-6)).repeat_interleave(H // G, dim=2)
+    q, k, v = unit(q.reshape(n_seq, T, G, d)) * d ** -0.5, unit(k.reshape(n_seq, T, G, d)), v.reshape(n_seq, T, H, d)
+    beta = torch.sigmoid(padded @ w["b"].T)
+    dt = torch.nn.functional.softplus((padded @ w["a1"].T) @ w["a2"].T + w["dt_bias"]).reshape(n_seq, T, H, d)
+    decay = torch.exp(-torch.exp(w["A_log"])[:, None] * dt)
+    gate = torch.sigmoid((padded @ w["g1"].T) @ w["g2"].T).reshape(n_seq, T, H, d)
+    S = torch.zeros(n_seq, H, d, d, dtype=torch.float64, device="cuda")
+    o = torch.empty(n_seq, T, H, d, dtype=torch.float64, device="cuda")
+    left = torch.tensor([a for a, _ in lens], device="cuda")
+    for s in range(T):
+        live = (s < left)[:, None, None, None]
+        N = decay[:, s, :, :, None] * S
+        u = beta[:, s, :, None] * (v[:, s] - torch.einsum("bhkv,bhk->bhv", N, k[:, s]))
+        N = N + k[:, s, :, :, None] * u[:, :, None, :]
+        o[:, s] = torch.einsum("bhkv,bhk->bhv", N, q[:, s])
+        S = torch.where(live, N, S)
+    o = (_rms(o, w["norm"]) * gate).reshape(n_seq, T, H * d) @ w["o"].T
+    last = torch.stack([before[i, a: a + TAPS - 1] for i, (a, _) in enumerate(lens)])
+    return [torch.cat([o[i, :a] for i, (a, _) in enumerate(lens)]), S, last]
