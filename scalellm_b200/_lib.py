@@ -272,7 +272,7 @@ def ensure(sources) -> C.CDLL:
     key = hashlib.sha1(" ".join(srcs).encode()).hexdigest()[:10]
     out = os.path.join(_HERE, f"libb200part-{key}.so")
     csrc = os.path.join(_HERE, "csrc")
-    deps = [os.path.join(csrc, s) for s in srcs] + [os.path.join(csrc, "common.cuh"),
+    deps = [os.path.join(csrc, s) for s in srcs] + [os.path.join(csrc, "common.cuh"), os.path.join(csrc, "guard.cuh"),
                                                     os.path.join(_HERE, "..", "include", "b200_decode.h")]
     import fcntl
     import subprocess

@@ -1,5 +1,5 @@
-// dense.cu — dense bf16 linear for decode-sized batches: C[M, N] = A[M, K] W[N, K]^T
-// (+ bias), M <= 128 rows per pass, replacing F::linear -> cuBLASLt
+// dense.cu — dense bf16 linear: C[M, N] = A[M, K] W[N, K]^T (+ bias), for decode-sized
+// batches (M <= 128 rows per pass, first kernel) and prompt-sized ones (second kernel), replacing F::linear -> cuBLASLt
 // (src/layers/linear/parallel_linear.cpp:256-263,294-308; lm_head models/meta/llama.h:259-265) for the
 // unquantised configuration and for lm_head.
 //
@@ -22,6 +22,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "guard.cuh"
 
 namespace b200 {
 
@@ -221,6 +222,211 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constan
 }
 
 // ---------------------------------------------------------------------------------------------
+// Prompt-sized batches: one pass over W, no partials.
+//
+// C^T tile = W tile x A tile^T on a PAIR of SMs (tcgen05.mma.cta_group::2, M = 256 output features x N = bt tokens):
+// each CTA of the pair stages its own 128 features and its own half of the tokens, so a k step of 64 moves
+// 16 KB + bt * 64 B per SM for 2 * bt tensor cycles — half the operand traffic per FLOP of a one-SM tile, which is what
+// bounds 128-row passes (they also re-read W once per pass and round-trip fp32 partials through HBM).  Features are the
+// M dimension because weights come in multiples of 256 rows while batches do not: the token tile bt takes any multiple
+// of 32 up to 256, chosen per call so that the last wave of pairs is full (dp_pick_bt).
+//   warp 0 TMA producer (both CTAs; bytes are counted on the leader's barrier), warp 1 of the leader MMA issuer,
+//   warps 4-7 epilogue: TMEM -> bf16 -> [32 tokens][128 features] in shared memory -> TMA store (clips M and N).
+// Accumulators are double buffered in TMEM (2 x 256 columns), so the epilogue of a tile runs under the next one's MMAs.
+// Bound by the tensor pipe: 4096 x 28672 with 1 999 rows 315 us = 1 489 TFLOP/s, 0.90 of the measured burst rate (128-row
+// passes: 922 us); 14336 x 4096 with 1 999 rows 161 us (553); where N gives few tiles, by the tiles' own length.
+// ---------------------------------------------------------------------------------------------
+constexpr int DP_STAGES = 6;
+constexpr int DP_HALF = 16384;                           // one operand of one stage: [128 x 64] bf16
+constexpr int DP_CHUNK = 32;                             // tokens per store
+constexpr int DP_OUT = DP_CHUNK * 128 * 2;               // staged output chunk
+constexpr int DP_THREADS = 8 * 32;
+constexpr size_t DP_SMEM = 1024 + (size_t)DP_STAGES * 2 * DP_HALF + 2 * DP_OUT + (2 * DP_STAGES + 4) * 8 + 64;
+
+struct DensePromptParams {
+  const __nv_bfloat16* bias;
+  int N, KB, bt, n_tt, tiles;       // KB: k steps of 64; n_tt: token tiles; tiles: feature tiles x token tiles
+};
+
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ uint32_t map_to_rank(uint32_t smem_addr, uint32_t rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_addr), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// load of this CTA's half tile; the bytes count on a barrier of the pair's leader
+__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
+      ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1) : "memory");
+}
+__device__ __forceinline__ void umma_bf16_pair(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+      ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(acc) : "memory");
+}
+// arrives on the barrier at this offset in both CTAs when the issued MMAs are done
+__device__ __forceinline__ void umma_commit_pair(uint32_t bar) {
+  asm volatile(
+      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+      ::"r"(bar), "h"((uint16_t)3) : "memory");
+}
+
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(DP_THREADS, 1)
+dense_prompt_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap amap,
+                    const __grid_constant__ CUtensorMap cmap, const DensePromptParams p) {
+  extern __shared__ uint8_t smem_dyn[];
+  uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~static_cast<uintptr_t>(1023));
+  uint8_t* w_smem = base;                                   // [stage][128 features x 64 k]
+  uint8_t* a_smem = w_smem + DP_STAGES * DP_HALF;           // [stage][bt / 2 tokens x 64 k]
+  uint8_t* o_smem = a_smem + DP_STAGES * DP_HALF;           // 2 x [32 tokens][128 features]
+  uint64_t* full = reinterpret_cast<uint64_t*>(o_smem + 2 * DP_OUT);   // used in the leader
+  uint64_t* empty = full + DP_STAGES;                       // in both: the stage's MMAs are done
+  uint64_t* tmem_full = empty + DP_STAGES;                  // in both
+  uint64_t* tmem_empty = tmem_full + 2;                     // in the leader: 4 epilogue warps of each CTA
+  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(tmem_empty + 2);
+  volatile uint32_t* dead = tmem_holder + 1;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t rank = cluster_rank();
+  const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
+
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < DP_STAGES; ++i) {
+      mbar_init(&full[i], 1);
+      mbar_init(&empty[i], 1);
+    }
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&tmem_full[i], 1);
+      mbar_init(&tmem_empty[i], 8);
+    }
+    *dead = 0u;
+    fence_mbar_init();
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(tmem_holder)) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+  }
+  if (warp == 0 && lane == 0) {
+    prefetch_tensormap(&wmap);
+    prefetch_tensormap(&amap);
+    prefetch_tensormap(&cmap);
+  }
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_holder;
+
+  if (warp == 0) {
+    if (lane == 0) {
+      pdl_wait();
+      const uint32_t half = (uint32_t)p.bt * 64;            // bytes of this CTA's token half: bt / 2 rows of 128 B
+      int cnt = 0;
+      for (int tile = pair; tile < p.tiles; tile += n_pairs) {
+        const int ft = tile / p.n_tt, tt = tile - ft * p.n_tt;
+        const int f0 = ft * 256 + (int)rank * 128, m0 = tt * p.bt + (int)rank * (p.bt >> 1);
+        for (int kb = 0; kb < p.KB; ++kb, ++cnt) {
+          const int s = cnt % DP_STAGES;
+          guard_wait(&empty[s], ((cnt / DP_STAGES) & 1) ^ 1, dead);
+          if (rank == 0) mbar_arrive_expect_tx(&full[s], 2 * (DP_HALF + half));
+          const uint32_t bar = map_to_rank(smem_u32(&full[s]), 0);
+          tma_load_2d_pair(smem_u32(w_smem + s * DP_HALF), &wmap, bar, kb * 64, f0);
+          tma_load_2d_pair(smem_u32(a_smem + s * DP_HALF), &amap, bar, kb * 64, m0);
+        }
+      }
+      for (int i = cnt > DP_STAGES ? cnt - DP_STAGES : 0; i < cnt; ++i)   // no arrival is under way when the pair ends
+        guard_wait(&empty[i % DP_STAGES], (i / DP_STAGES) & 1, dead);
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    if (rank == 0) {
+      const uint32_t idesc = umma_idesc_bf16(256, (uint32_t)p.bt);
+      const uint32_t w_base = smem_u32(w_smem), a_base = smem_u32(a_smem);
+      int cnt = 0, it = 0;
+      for (int tile = pair; tile < p.tiles; tile += n_pairs, ++it) {
+        const int buf = it & 1;
+        guard_wait(&tmem_empty[buf], ((it >> 1) & 1) ^ 1, dead);
+        tc_fence_after();
+        for (int kb = 0; kb < p.KB; ++kb, ++cnt) {
+          const int s = cnt % DP_STAGES;
+          guard_wait(&full[s], (cnt / DP_STAGES) & 1, dead);
+          tc_fence_after();
+          if (elect_one()) {
+            const uint64_t wd = umma_desc_kmajor_sw128(w_base + s * DP_HALF);
+            const uint64_t ad = umma_desc_kmajor_sw128(a_base + s * DP_HALF);
+#pragma unroll
+            for (int ks = 0; ks < 4; ++ks)                  // 16 k = 32 bytes inside the swizzled rows
+              umma_bf16_pair(tmem_base + buf * 256, wd + ks * 2, ad + ks * 2, idesc, (kb > 0 || ks > 0) ? 1u : 0u);
+            umma_commit_pair(smem_u32(&empty[s]));
+            if (kb == p.KB - 1) umma_commit_pair(smem_u32(&tmem_full[buf]));
+          }
+          __syncwarp();
+        }
+      }
+    }
+    __syncwarp();
+  } else if (warp >= 4) {
+    const int quad = warp & 3, et = threadIdx.x - 128;
+    pdl_wait();                                             // C may still be read by an earlier kernel
+    int it = 0, chunk = 0;
+    for (int tile = pair; tile < p.tiles; tile += n_pairs, ++it) {
+      const int ft = tile / p.n_tt, tt = tile - ft * p.n_tt, buf = it & 1;
+      const int f0 = ft * 256 + (int)rank * 128, f = f0 + et;
+      const bool has_bias = p.bias != nullptr;
+      const float bias = has_bias && f < p.N ? __bfloat162float(p.bias[f]) : 0.0f;
+      guard_wait(&tmem_full[buf], (it >> 1) & 1, dead);
+      tc_fence_after();
+      const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + buf * 256;
+      for (int c0 = 0; c0 < p.bt; c0 += DP_CHUNK, ++chunk) {
+        uint32_t r[32];
+        tmem_ld_32x32b_x32(taddr + c0, r);
+        tmem_ld_wait();
+        if (c0 + DP_CHUNK >= p.bt) {                        // the accumulator is in registers: hand it back
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0)
+            asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(
+                             map_to_rank(smem_u32(&tmem_empty[buf]), 0)) : "memory");
+        }
+        if (et == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+        asm volatile("bar.sync 1, 128;" ::: "memory");      // the staging buffer of two chunks ago has been read
+        const bool lost = *dead != 0u;
+        __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(o_smem + (chunk & 1) * DP_OUT) + et;
+#pragma unroll
+        for (int i = 0; i < 32; ++i) {
+          __nv_bfloat16 v = __float2bfloat16_rn(lost ? NAN : __uint_as_float(r[i]));
+          if (has_bias) v = __float2bfloat16_rn(__bfloat162float(v) + bias);
+          o[i * 128] = v;
+        }
+        fence_proxy_async_smem();
+        asm volatile("bar.sync 1, 128;" ::: "memory");
+        if (et == 0) {
+          asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];"
+                       ::"l"(&cmap), "r"(smem_u32(o_smem + (chunk & 1) * DP_OUT)), "r"(f0), "r"(tt * p.bt + c0)
+                       : "memory");
+          asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+        }
+      }
+    }
+    if (et == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+  }
+  if (warp == 0 && lane == 0 && *dead) guard_drain();
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync();                                           // the peer's barriers and tensor memory stay until both are done
+  if (warp == 1)
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, 512;" ::"r"(tmem_base) : "memory");
+}
+
+// ---------------------------------------------------------------------------------------------
 // host
 // ---------------------------------------------------------------------------------------------
 struct DMapKey {
@@ -278,6 +484,73 @@ static int launch_dense(const CUtensorMap& wmap, const CUtensorMap& amap, const 
   return B200_OK;
 }
 
+// Which kernel: above 128 rows the partials kernel re-reads W per 128 rows (4096 x 28672, 1 999 rows: 922 us against 315;
+// 14336 x 4096, 129 rows: 60 against 57).  Below, it streams W from all SMs whatever N is, where the one-pass kernel has
+// only one tile per 256 features (14336 x 4096, 128 rows: 36 against 57) — but pays a reduction launch and, from 64 rows,
+// operand traffic: with whole waves of feature tiles the one-pass kernel is ahead from about 64 rows (4096 x 28672, 96
+// rows: 56 against 50), with many waves from about 40 (4096 x 128256: 32 rows 170 against 172, 48 rows 178 against 175,
+// 64 rows 183 against 177).
+static bool dp_taken(int64_t M, int64_t N, int64_t n_pairs) {
+  const int64_t n_ft = (N + 255) / 256;
+  return M > 128 || (M > 64 && n_ft >= n_pairs) || (M > 40 && n_ft >= 4 * n_pairs);
+}
+
+// Token tile: waves of SM pairs x (tensor or operand-traffic cycles of a k step, whichever is longer) over all tile
+// sizes; a smaller tile costs operand traffic per FLOP, a larger one padding or a last wave that is nearly empty.
+static int dp_pick_bt(int64_t M, int64_t N, int64_t K, int n_pairs) {
+  const int64_t n_ft = (N + 255) / 256, kb = K / 64;
+  int best = 256;
+  double best_cost = 0.0;
+  for (int bt = 256; bt >= 32; bt -= 32) {
+    const int64_t waves = (n_ft * ((M + bt - 1) / bt) + n_pairs - 1) / n_pairs;
+    const double step = 2.0 * bt, traffic = (DP_HALF + bt * 64) / 64.0;
+    const double cost = (double)waves * ((double)kb * (step > traffic ? step : traffic) + 1000.0);
+    if (bt == 256 || cost < best_cost) {
+      best = bt;
+      best_cost = cost;
+    }
+  }
+  return best;
+}
+
+static int encode_2d(CUtensorMap* m, const void* ptr, int64_t cols, int64_t rows, int64_t ld, int box_cols, int box_rows,
+                     bool swizzle) {
+  tensor_map_encode_fn enc = get_tensor_map_encode();
+  if (!enc) return set_error(B200_ERR_CUDA, "cuTensorMapEncodeTiled entry point unavailable");
+  cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
+  cuuint64_t strides[1] = {(cuuint64_t)ld * 2};
+  cuuint32_t box[2] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows};
+  cuuint32_t estr[2] = {1, 1};
+  CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), dims, strides, box, estr,
+                   CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
+                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return set_error(B200_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d) for a dense operand", (int)r);
+  return B200_OK;
+}
+
+static int launch_dense_prompt(void* C, const void* A, const void* W, const void* bias, int64_t M, int64_t N, int64_t K,
+                               int64_t lda, int64_t ldw, int64_t ldc, cudaStream_t st) {
+  const int n_pairs = sm_count() / 2;
+  const int bt = dp_pick_bt(M, N, K, n_pairs);
+  CUtensorMap wmap, amap, cmap;
+  int rc = encode_2d(&wmap, W, K, N, ldw, 64, 128, true);
+  if (rc == B200_OK) rc = encode_2d(&amap, A, K, M, lda, 64, bt / 2, true);
+  if (rc == B200_OK) rc = encode_2d(&cmap, C, N, M, ldc, 128, DP_CHUNK, false);
+  if (rc != B200_OK) return rc;
+  DensePromptParams p{};
+  p.bias = static_cast<const __nv_bfloat16*>(bias);
+  p.N = (int)N;
+  p.KB = (int)(K / 64);
+  p.bt = bt;
+  p.n_tt = (int)((M + bt - 1) / bt);
+  const int64_t tiles = (N + 255) / 256 * p.n_tt;
+  p.tiles = (int)tiles;
+  B200_CUDA_OK(cudaFuncSetAttribute(dense_prompt_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DP_SMEM));
+  const unsigned grid = 2u * (unsigned)(tiles < n_pairs ? tiles : n_pairs);
+  B200_PDL_LAUNCH_L(1, "dense_prompt", dense_prompt_kernel, grid, DP_THREADS, DP_SMEM, st, wmap, amap, cmap, p);
+  return B200_OK;
+}
+
 }  // namespace b200
 
 using namespace b200;
@@ -303,6 +576,9 @@ int b200_dense_gemm(void* C, const void* A, const void* W, const void* bias, int
   if (M == 0) return B200_OK;
   B200_CHECK_ARG(workspace && is_aligned(workspace, 16), "dense_gemm: workspace required");
   auto st = static_cast<cudaStream_t>(stream);
+  // the one-pass kernel stores C by TMA: rows on 16 bytes
+  if (dp_taken(M, N, sm_count() / 2) && ldc % 8 == 0 && is_aligned(C, 16) && M < (1ll << 31) && N < (1ll << 31))
+    return launch_dense_prompt(C, A, W, bias, M, N, K, lda, ldw, ldc, st);
   const W4Plan plan = w4_get_plan(up128(N), up128(K), 128);   // one weight tile per unit
   CUtensorMap wmap;
   int rc = get_kmajor_map(DMapKey{W, N, K, ldw, 128}, &wmap);

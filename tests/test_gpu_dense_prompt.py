@@ -1,0 +1,31 @@
+"""The one-pass dense kernel for prompt-sized batches (csrc/dense.cu) against 64-bit products: edges of the token tile, of
+the pair's 256 features and of the k step, strided rows, a column block of a wider result, the bias."""
+import pytest
+import torch
+
+from scalellm_b200 import kernels
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("M,N,K", [(129, 8, 64), (129, 136, 128), (160, 256, 4096), (257, 264, 192), (300, 1000, 448),
+                                   (513, 4096, 1024), (2048, 20480, 64), (1999, 6144, 512), (65, 18944, 128),
+                                   (41, 75776, 64)])
+@pytest.mark.parametrize("bias", [False, True])
+def test_against_64_bits(M, N, K, bias):
+    g = torch.Generator(device="cuda").manual_seed(M * 7 + N + K)
+    rnd = lambda *s: torch.randn(s, generator=g, device="cuda").to(torch.bfloat16)
+    a, w = rnd(M, K + 24)[:, 8: 8 + K], rnd(N, K + 8)[:, :K]
+    b = rnd(N) if bias else None
+    wide = torch.full((M + 2, N + 16), 7.0, dtype=torch.bfloat16, device="cuda")
+    out = wide[1: 1 + M, 8: 8 + N]
+    kernels.dense_gemm(a, w, b, out=out)
+    ref = a.double() @ w.double().T
+    # one rounding to 8 significant bits (at most 2^-8 of the value, twice with a bias), fp32 sums of K products (K 2^-24 of the sum of magnitudes)
+    err = 2.0 ** -8 * ref.abs() + K * 2.0 ** -24 * (a.double().abs() @ w.double().abs().T)
+    if bias:
+        ref = ref + b.double()
+        err = err + 2.0 ** -8 * (ref.abs() + err)
+    assert bool(((out.double() - ref).abs() <= err * 1.01 + 1e-30).all())
+    wide[1: 1 + M, 8: 8 + N] = 7.0
+    assert bool((wide == 7.0).all())               # nothing outside the block was written
