@@ -522,6 +522,34 @@ B200_API int b200_latent_attn(void* out, int64_t out_head_stride, int64_t out_to
  * separate CTAs and are merged by a second kernel (n_splits > 1 needs the workspace below); n_splits = 0: the
  * CUDA-core form (any dtype, fp32 arithmetic throughout). */
 B200_API int64_t b200_latent_attn_workspace_bytes(int64_t rows, int64_t H, int64_t rank, int64_t n_splits);
+/* Prompt portions on the tensor cores over keys and values that lie in order (prompt_attn.cu).  gather: paged rows
+ * (bf16, one or two caches [slots, cols] with row strides ld) in order; sequence i starts at row cu_block_lens[i] *
+ * block_size + 16 i and ends in at least 16 rows of zeros.  attn: q (fp32 or bf16, heads of 128, or of 192 with k_shared:
+ * the last 64 key channels of all heads) over rows laid out so; values of 128; H / G query heads per key head (a divisor of
+ * 128); r1 / r2 / sink / gate / out_mul / window as for b200_sink_attn (no r1 with k_shared); scale > 0; rows on 16 bytes. */
+B200_API int b200_prompt_gather(void* dst0, const void* src0, int64_t ld0, int64_t cols0, void* dst1 /*nullable*/,
+                                const void* src1, int64_t ld1, int64_t cols1, const int32_t* kv_cu_lens,
+                                const int32_t* block_tables, const int32_t* cu_block_lens, int64_t n_seq, int64_t kv_max,
+                                int64_t block_size, b200_stream_t stream);
+B200_API int b200_prompt_attn(void* out, int64_t out_token_stride, int64_t out_head_stride, const void* q,
+                              int64_t q_token_stride, int64_t q_head_stride, int q_is_fp32, const void* k, int64_t ldk,
+                              int64_t k_head_stride, const void* k_shared /*nullable*/, int64_t ld_shared, const void* v,
+                              int64_t ldv, int64_t v_head_stride, int64_t n_key_rows, const float* r1 /*nullable*/,
+                              const float* r2 /*nullable*/, const float* sink /*nullable*/, const void* gate /*nullable*/,
+                              int64_t ld_gate, float out_mul, int gate_heads, int64_t window, const int32_t* q_cu_lens,
+                              const int32_t* kv_cu_lens, const int32_t* cu_block_lens, int64_t n_seq, int64_t q_max,
+                              int64_t H, int64_t G, int64_t block_size, float scale, b200_stream_t stream);
+/* Both for dense caches [slots, G, 128]: q [rows, H, 128]; the workspace takes the ordered rows (n_key_rows: table entries *
+ * block_size + 16 n_seq).  k_cache == v_cache: the values are the keys. */
+B200_API int64_t b200_prompt_attn_paged_workspace_bytes(int64_t n_key_rows, int64_t G, int shared_kv);
+B200_API int b200_prompt_attn_paged(void* out, int64_t ldo, const void* q, int q_is_fp32, const void* k_cache,
+                                    const void* v_cache, void* workspace, int64_t workspace_bytes, int64_t n_key_rows,
+                                    const float* r1 /*nullable*/, const float* r2 /*nullable*/, const float* sink /*nullable*/,
+                                    const void* gate /*nullable*/, int64_t ld_gate, float out_mul, int gate_heads,
+                                    int64_t window, const int32_t* q_cu_lens, const int32_t* kv_cu_lens,
+                                    const int32_t* block_tables, const int32_t* cu_block_lens, int64_t n_seq, int64_t q_max,
+                                    int64_t kv_max, int64_t H, int64_t G, int64_t block_size, float scale,
+                                    b200_stream_t stream);
 /* Generalised delta rule over each sequence's tokens of the step (see delta_rule.cu); r, k, v, removal and gate
  * logits are column blocks [H * d] of matrices with row stride ld, the decay logits have row stride ld_decay;
  * state fp32 [n_slots, H, d, d]. */

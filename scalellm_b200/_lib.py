@@ -107,6 +107,13 @@ SIGNATURES = {
     "b200_latent_attn": (_int, [_vp, _i64, _i64, _vp, _i64, _i64, _int, _vp, _i64, _vp, _i64, _vp, _vp, _vp,
                                 _vp, _vp, _i64, _i64, _i64, _i64, _i64, _i64, _f32, _i64, _int, _vp, _i64, _int, _vp]),
     "b200_latent_attn_workspace_bytes": (_i64, [_i64, _i64, _i64, _i64]),
+    "b200_prompt_gather": (_int, [_vp, _vp, _i64, _i64, _vp, _vp, _i64, _i64, _vp, _vp, _vp, _i64, _i64, _i64, _vp]),
+    "b200_prompt_attn": (_int, [_vp, _i64, _i64, _vp, _i64, _i64, _int, _vp, _i64, _i64, _vp, _i64, _vp, _i64, _i64, _i64,
+                                _vp, _vp, _vp, _vp, _i64, _f32, _int, _i64, _vp, _vp, _vp, _i64, _i64, _i64, _i64, _i64,
+                                _f32, _vp]),
+    "b200_prompt_attn_paged_workspace_bytes": (_i64, [_i64, _i64, _int]),
+    "b200_prompt_attn_paged": (_int, [_vp, _i64, _vp, _int, _vp, _vp, _vp, _i64, _i64, _vp, _vp, _vp, _vp, _i64, _f32, _int,
+                                      _i64, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _i64, _i64, _i64, _f32, _vp]),
     "b200_delta_rule": (_int, [_vp, _i64, _vp, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _vp, _vp, _vp, _vp, _vp,
                                _vp, _vp, _i64, _i64, _i64, _f32, _f32, _f32, _int, _vp]),
     "b200_moe_route": (_int, [_vp, _vp, _vp, _i64, _vp, _i64, _i64, _i64, _i64, _int, _vp]),
@@ -210,7 +217,7 @@ SIGNATURES = {
 # just the sources a model asks for into a library of its own.
 ALL_SOURCES = ("runtime.cu", "elementwise.cu", "sampling.cu", "paged_attn.cu", "prefill_attn.cu", "w4a16.cu",
                "dense.cu", "allreduce.cu", "hyper.cu", "latent_attn.cu", "delta_rule.cu", "moe.cu", "postnorm.cu", "mingru.cu",
-               "diff_attn.cu", "sink_attn.cu", "sigmoid_attn.cu", "filters.cu", "linear_scan.cu")
+               "diff_attn.cu", "sink_attn.cu", "sigmoid_attn.cu", "filters.cu", "linear_scan.cu", "prompt_attn.cu")
 
 _lib: Optional[C.CDLL] = None
 _lib_sources: frozenset = frozenset()

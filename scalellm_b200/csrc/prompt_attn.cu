@@ -1,0 +1,623 @@
+// prompt_attn.cu — causal softmax attention of prompt portions on the 5th-generation tensor cores, for heads of 128
+// value channels and queries and keys of 128 or 192 (128 plus a part of 64 that all heads share), over keys and values
+// that lie in order.  It serves the designs whose softmax weights enter the value product in more than 16 bits:
+//
+//     s_ij = scale q_i . k_j - r1_h ln(1 + r2_h (i - j))        j <= i, and i - j < window (window 0: all)
+//     o_i  = sum_j p_ij v_j,  p_ij = exp(s_ij) / (exp(sink_h) + sum_j' exp(s_ij'))
+//     what is stored: out_mul * o * sigmoid(gate)
+//
+//   gather  : the sequences' paged rows, in order, into one array; sequence i starts at row
+//             cu_block_lens[i] * block_size + 16 i and is followed by zeros up to at least 16 rows, so a 16-key step of
+//             the value product never meets another sequence's rows.  One pass over the keys (2 x their bytes) buys
+//             plain 128-row TMA tiles whatever the block size is: paged tiles cost 32 boxes each at 8 slots a block.
+//   attend  : one CTA per (sequence, key/value head, 2 x 128 query rows); a tile's rows are its tokens x the query heads
+//             of the key/value head.  Key tiles of 128.
+//
+// Warps 0-3 and 4-7 are two softmax groups, one per 128-row tile, a thread per row; warp 8 loads, warp 9 issues MMAs:
+//   S_w = Q_w K^T -> TMEM;  softmax group w turns S_w into weights IN PLACE, as two bf16 terms per weight (high and low
+//   part: 16 bits of mantissa, exactly the 128 fp32 columns' space);  O_w += P_hi V + P_lo V with P read from TMEM.
+// While one group works on its scores the tensor pipe runs the other tile's products (PV_0 S_0' PV_1 S_1' ...).  The
+// running maximum that O is relative to moves only when a row's maximum grows by more than 2^8 (a weight may then be up to
+// 2^8; its rounding is relative all the same), so O is almost never rescaled: it stays in TMEM until the end.
+//
+// Bound by the chain scores -> weights -> products of a tile: per 128 x 128 tile 2 x (64 NA + 256) x 128 x 128 FLOPs, where
+// the low parts are a third.  4 prompts of up to 2 048 tokens, 16 heads: 160 us with 192-wide keys (the kernel that attends in
+// the latent space: 3.9 ms), 138 us with bias and sink over 4 key heads (mma.sync kernel: 430 us).
+#include "common.cuh"
+#include "guard.cuh"
+
+namespace b200 {
+namespace {
+
+constexpr int PA_ROWS = 128, PA_KEYS = 128, PA_VD = 128;
+constexpr int PA_ATOM = 128 * 128;              // [128 rows x 64] bf16, 128-byte swizzle
+constexpr int PA_VHALF = 64 * 128 * 2;          // V of 64 keys: two [64 keys x 64] chunks
+constexpr int PA_THREADS = 12 * 32;             // two softmax warpgroups; loads, MMAs and two idle warps
+constexpr float PA_LOG2E = 1.4426950408889634f;
+constexpr float PA_SLACK = 8.0f;                // log2 of the growth of a row's maximum that is tolerated
+
+template <int NA>
+struct PaCfg {
+  static constexpr int KST = 2;                 // key tiles in flight
+  static constexpr int NV = NA == 3 ? 2 : 4;    // halves of value tiles in flight
+  static constexpr int TILES = (2 * NA + KST * NA + NV) * PA_ATOM;
+  static constexpr int BARS = 1 + 2 * KST + 2 * NV + 6;
+};
+
+struct PromptAttnParams {
+  __nv_bfloat16* out;
+  int64_t out_ts, out_hs;
+  const void* q;
+  int64_t q_ts, q_hs;
+  const int *q_cu, *kv_cu, *blk_cu;
+  const float *r1, *r2, *sink;
+  const __nv_bfloat16* gate;
+  int64_t ld_gate;
+  float out_mul, scale_log2;
+  int gate_heads, gate_vec, block_size, per, per_log2, window, q_blocks;
+  int k_hs, v_hs, tab_ld;                       // columns between key heads / value heads; bias table row
+};
+
+__device__ __forceinline__ float pa_ex2(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+// two fp32 operations an instruction
+__device__ __forceinline__ float2 pa_fma2(float2 a, float2 b, float2 c) {
+  float2 d;
+  asm("{\n\t.reg .b64 ra, rb, rc, rd;\n\tmov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %5};\n\tmov.b64 rc, {%6, %7};\n\t"
+      "fma.rn.f32x2 rd, ra, rb, rc;\n\tmov.b64 {%0, %1}, rd;\n\t}"
+      : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return d;
+}
+__device__ __forceinline__ float2 pa_add2(float2 a, float2 b) {
+  float2 d;
+  asm("{\n\t.reg .b64 ra, rb, rd;\n\tmov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %5};\n\t"
+      "add.rn.f32x2 rd, ra, rb;\n\tmov.b64 {%0, %1}, rd;\n\t}"
+      : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return d;
+}
+__host__ __device__ constexpr uint32_t pa_idesc(uint32_t N, uint32_t b_mn) {
+  return umma_idesc_bf16(128, N) | (b_mn << 16);
+}
+// [8 keys x 64 channels] atoms, channels contiguous: 64-channel chunks 8 KB apart, 8-key groups 1 KB apart
+__device__ __forceinline__ uint64_t pa_desc_v(uint32_t smem_addr) {
+  return static_cast<uint64_t>((smem_addr & 0x3ffffu) >> 4) | static_cast<uint64_t>(8192 >> 4) << 16 |
+         static_cast<uint64_t>(1024 >> 4) << 32 | static_cast<uint64_t>(1) << 46 | static_cast<uint64_t>(2) << 61;
+}
+__device__ __forceinline__ void pa_st16(uint32_t taddr, const uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
+      ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]),
+        "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]) : "memory");
+}
+
+template <int NA, bool BIAS, typename QT>
+__global__ void __launch_bounds__(PA_THREADS, 1)
+prompt_attn_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__ CUtensorMap rmap,
+                   const __grid_constant__ CUtensorMap vmap, const PromptAttnParams p) {
+  using Cfg = PaCfg<NA>;
+  extern __shared__ uint8_t smem_dyn[];
+  const int g = blockIdx.x, seq = blockIdx.y, qb = p.q_blocks - 1 - (int)blockIdx.z;   // long walks first
+  const int tpb = PA_ROWS >> p.per_log2;
+  const int q_begin = p.q_cu[seq], q_len = p.q_cu[seq + 1] - q_begin;
+  const int t0 = qb * 2 * tpb;
+  if (t0 >= q_len) return;
+  const int kv_len = p.kv_cu[seq + 1] - p.kv_cu[seq];
+  const int key0 = p.blk_cu[seq] * p.block_size + 16 * seq;
+  // per row tile: its tokens, positions and key tiles [lo, hi)
+  int n_tok[2], pos0[2], lo[2], hi[2];
+#pragma unroll
+  for (int w = 0; w < 2; ++w) {
+    n_tok[w] = min(max(q_len - t0 - w * tpb, 0), tpb);
+    pos0[w] = kv_len - q_len + t0 + w * tpb;
+    lo[w] = (p.window > 0 ? max(0, pos0[w] - p.window + 1) : 0) / PA_KEYS;
+    hi[w] = n_tok[w] > 0 ? (pos0[w] + n_tok[w] - 1) / PA_KEYS + 1 : 0;
+    if (n_tok[w] <= 0) lo[w] = 0;
+  }
+  const int i0 = lo[0], i1 = max(hi[0], hi[1]);            // (tile 1 starts no earlier than tile 0 and ends no earlier)
+
+  uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~static_cast<uintptr_t>(1023));
+  uint8_t* q_smem = base;                                  // [2][NA] atoms
+  uint8_t* k_smem = q_smem + 2 * NA * PA_ATOM;             // [KST][NA] atoms
+  uint8_t* v_smem = k_smem + Cfg::KST * NA * PA_ATOM;      // [NV] halves
+  uint64_t* bars = reinterpret_cast<uint64_t*>(base + Cfg::TILES);
+  uint64_t* q_full = bars;
+  uint64_t* k_full = bars + 1;
+  uint64_t* k_empty = k_full + Cfg::KST;
+  uint64_t* v_full = k_empty + Cfg::KST;
+  uint64_t* v_empty = v_full + Cfg::NV;
+  uint64_t* s_full = v_empty + Cfg::NV;                    // [2]
+  uint64_t* p_full = s_full + 2;                           // [2]
+  uint64_t* o_full = p_full + 2;                           // [2]
+  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(bars + Cfg::BARS);
+  volatile uint32_t* dead = tmem_holder + 1;
+  float* tab = reinterpret_cast<float*>(tmem_holder + 4);  // [2 groups][2][per][tab_ld] (distance bias)
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+
+  if (threadIdx.x == 0) {
+    mbar_init(q_full, 8);
+    for (int i = 0; i < Cfg::KST; ++i) { mbar_init(&k_full[i], 1); mbar_init(&k_empty[i], 1); }
+    for (int i = 0; i < Cfg::NV; ++i) { mbar_init(&v_full[i], 1); mbar_init(&v_empty[i], 1); }
+    for (int i = 0; i < 2; ++i) { mbar_init(&s_full[i], 1); mbar_init(&p_full[i], 4); mbar_init(&o_full[i], 1); }
+    *dead = 0u;
+    fence_mbar_init();
+  }
+  if (warp == 9) {
+    tmem_alloc(tmem_holder, 512);
+    tmem_relinquish();
+  }
+  if (warp == 8 && lane == 0) {
+    prefetch_tensormap(&kmap);
+    if (NA == 3) prefetch_tensormap(&rmap);
+    prefetch_tensormap(&vmap);
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *tmem_holder;                      // S_0 | S_1 | O_0 | O_1, 128 columns each
+
+  // 384 threads x 168 registers at launch = 256 x 200 + 128 x 104: a softmax thread holds its row's 128 scores
+  if (warp >= 8) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 104;");
+    if (warp == 8) {
+      if (lane == 0) {
+        for (int i = i0; i < i1; ++i) {
+          const int n = i - i0, s = n % Cfg::KST, row = key0 + i * PA_KEYS;
+          guard_wait(&k_empty[s], ((n / Cfg::KST) & 1) ^ 1, dead);
+          mbar_arrive_expect_tx(&k_full[s], NA * PA_ATOM);
+          uint8_t* kd = k_smem + s * NA * PA_ATOM;
+          tma_load_2d(kd, &kmap, &k_full[s], g * p.k_hs, row);
+          tma_load_2d(kd + PA_ATOM, &kmap, &k_full[s], g * p.k_hs + 64, row);
+          if (NA == 3) tma_load_2d(kd + 2 * PA_ATOM, &rmap, &k_full[s], 0, row);
+#pragma unroll
+          for (int half = 0; half < 2; ++half) {
+            const int nv = 2 * n + half, sv = nv % Cfg::NV;
+            guard_wait(&v_empty[sv], ((nv / Cfg::NV) & 1) ^ 1, dead);
+            mbar_arrive_expect_tx(&v_full[sv], PA_VHALF);
+            uint8_t* vd = v_smem + sv * PA_VHALF;
+            tma_load_2d(vd, &vmap, &v_full[sv], g * p.v_hs, row + half * 64);
+            tma_load_2d(vd + PA_VHALF / 2, &vmap, &v_full[sv], g * p.v_hs + 64, row + half * 64);
+          }
+        }
+      }
+      __syncwarp();
+    } else if (warp == 9) {
+      // (the whole warp walks the loop and one elected lane issues: descriptors stay in uniform registers)
+      const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
+      const uint64_t qd = umma_desc_kmajor_sw128(__shfl_sync(0xffffffffu, smem_u32(q_smem), 0));
+      const uint64_t kd = umma_desc_kmajor_sw128(__shfl_sync(0xffffffffu, smem_u32(k_smem), 0));
+      const uint64_t vd = pa_desc_v(__shfl_sync(0xffffffffu, smem_u32(v_smem), 0));
+      auto in_range = [&](int w, int i) { return i >= lo[w] && i < hi[w]; };
+      auto scores = [&](int w, int i) {
+        const uint64_t a = qd + w * (NA * PA_ATOM >> 4), b = kd + ((i - i0) % Cfg::KST) * (NA * PA_ATOM >> 4);
+        if (elect_one()) {
+#pragma unroll
+          for (int ks = 0; ks < NA * 4; ++ks) {
+            constexpr uint32_t idesc = pa_idesc(128, 0);
+            const uint32_t off = ((ks >> 2) * PA_ATOM + (ks & 3) * 32) >> 4;
+            umma_bf16(tm + w * 128, a + off, b + off, idesc, ks > 0 ? 1u : 0u);
+          }
+          umma_commit(&s_full[w]);
+        }
+        __syncwarp();
+      };
+      auto key_tile = [&](int i) {
+        guard_wait(&k_full[(i - i0) % Cfg::KST], ((i - i0) / Cfg::KST) & 1, dead);
+        tc_fence_after();
+      };
+      auto commit = [&](uint64_t* bar) {
+        if (elect_one()) umma_commit(bar);
+        __syncwarp();
+      };
+      guard_wait(q_full, 0, dead);
+      int done[2] = {0, 0};                                // weight tiles taken of each row tile
+      key_tile(i0);
+#pragma unroll
+      for (int w = 0; w < 2; ++w)
+        if (in_range(w, i0)) scores(w, i0);
+      commit(&k_empty[0]);
+      for (int i = i0; i < i1; ++i) {
+        const int last = in_range(1, i) ? 1 : 0;           // the last row tile that reads V(i)
+        bool k_ready = false;
+#pragma unroll
+        for (int w = 0; w < 2; ++w) {
+          if (in_range(w, i)) {
+            guard_wait(&p_full[w], done[w] & 1, dead);
+            tc_fence_after();
+            const int steps = min(8, (pos0[w] + n_tok[w] - i * PA_KEYS + 15) >> 4);   // 16-key steps with visible keys
+            const uint32_t o = tm + 256 + w * 128, pw = tm + w * 128;
+            constexpr uint32_t idesc = pa_idesc(PA_VD, 1);
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+              const int nv = 2 * (i - i0) + half, sv = nv % Cfg::NV;
+              if (w == 0 || !in_range(0, i)) {
+                guard_wait(&v_full[sv], (nv / Cfg::NV) & 1, dead);
+                tc_fence_after();
+              }
+              const uint64_t v = vd + sv * (PA_VHALF >> 4);
+              const uint32_t acc = done[w] > 0 || half > 0 ? 1u : 0u;
+              const int n_steps = steps - half * 4;
+              if (elect_one()) {
+#pragma unroll
+                for (int kk = 0; kk < 4; ++kk)
+                  if (kk < n_steps) {
+                    umma_bf16_ts(o, pw + (half * 4 + kk) * 8, v + kk * 128, idesc, kk > 0 ? 1u : acc);
+                    umma_bf16_ts(o, pw + 64 + (half * 4 + kk) * 8, v + kk * 128, idesc, 1u);
+                  }
+                if (w == last) umma_commit(&v_empty[sv]);
+                if (half == 1 && i + 1 == hi[w]) umma_commit(&o_full[w]);
+              }
+              __syncwarp();
+            }
+            ++done[w];
+          }
+          if (in_range(w, i + 1)) {
+            if (!k_ready) key_tile(i + 1);
+            k_ready = true;
+            scores(w, i + 1);
+          }
+        }
+        if (k_ready) commit(&k_empty[(i + 1 - i0) % Cfg::KST]);
+      }
+    }
+  } else {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 200;");
+    const int w = warp >> 2, r = threadIdx.x & 127;        // this thread's row of tile w
+    const int tok = r >> p.per_log2, hh = r & (p.per - 1), h = g * p.per + hh;
+    const bool live = tok < n_tok[w];
+    const uint32_t lane_off = (uint32_t)((warp & 3) * 32) << 16;
+    // Q: a warp stages its 32 rows, 4 channels a lane, as the K-major swizzled operand
+    {
+      uint8_t* qt = q_smem + w * NA * PA_ATOM;
+      constexpr int PER = (NA * 64 + 127) / 128, BATCH = 16;   // pieces of a row a lane loads; rows in flight
+#pragma unroll 1
+      for (int j0 = 0; j0 < 32; j0 += BATCH) {
+        float v[BATCH][PER][4];
+#pragma unroll
+        for (int j = 0; j < BATCH; ++j) {
+          const int rr = (warp & 3) * 32 + j0 + j, tk = rr >> p.per_log2, hq = g * p.per + (rr & (p.per - 1));
+          const QT* src = static_cast<const QT*>(p.q) + (int64_t)(q_begin + t0 + w * tpb + tk) * p.q_ts + (int64_t)hq * p.q_hs;
+#pragma unroll
+          for (int c = 0; c < PER; ++c) {
+            const int d = lane * 4 + c * 128;
+            v[j][c][0] = v[j][c][1] = v[j][c][2] = v[j][c][3] = 0.0f;
+            if (tk < n_tok[w] && d < NA * 64) load4<QT>(src + d, v[j][c]);
+          }
+        }
+#pragma unroll
+        for (int j = 0; j < BATCH; ++j) {
+          const int rr = (warp & 3) * 32 + j0 + j;
+#pragma unroll
+          for (int c = 0; c < PER; ++c) {
+            const int d = lane * 4 + c * 128;
+            if (d < NA * 64) {
+              uint2 pk;
+              pk.x = Num<__nv_bfloat16>::pack(v[j][c][0], v[j][c][1]);
+              pk.y = Num<__nv_bfloat16>::pack(v[j][c][2], v[j][c][3]);
+              const int piece = (d & 63) >> 3;             // 16-byte piece of the row's 128 bytes
+              *reinterpret_cast<uint2*>(qt + (d >> 6) * PA_ATOM + rr * 128 + ((piece ^ (rr & 7)) << 4) + (d & 4) * 2) = pk;
+            }
+          }
+        }
+      }
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(q_full);
+    }
+    const int pos = pos0[w] + tok;
+    const int first = p.window > 0 ? max(0, pos - p.window + 1) : 0;     // the row's first visible key
+    const uint32_t s_col = tmem + w * 128 + lane_off, o_col = tmem + 256 + w * 128 + lane_off;
+    float m = -INFINITY, l = 0.0f;                         // (log2 domain) what O and l are relative to; sum of weights
+    int n = 0;
+    for (int i = lo[w]; i < hi[w]; ++i, ++n) {
+      const int k0 = i * PA_KEYS;
+      const float* tb = nullptr;
+      if (BIAS) {
+        float* t = tab + (w * 2 + (n & 1)) * p.per * p.tab_ld;
+        const int d0 = pos0[w] - k0 - (PA_KEYS - 1);       // distance of table entry 0
+        for (int e = r; e < p.per * p.tab_ld; e += 128) {
+          const int eh = e / p.tab_ld, ed = e - eh * p.tab_ld;
+          const float b1 = p.r1[g * p.per + eh], b2 = p.r2[g * p.per + eh];
+          t[e] = -b1 * PA_LOG2E * logf(1.0f + b2 * (float)(d0 + ed));
+        }
+        asm volatile("bar.sync %0, 128;" ::"r"(1 + w) : "memory");
+        tb = t + hh * p.tab_ld + tok + PA_KEYS - 1;        // tb[-e]: the bias of key k0 + e
+      }
+      guard_wait(&s_full[w], n & 1, dead);
+      tc_fence_after();
+      float s[PA_KEYS];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        uint32_t u[32];
+        tmem_ld_32x32b_x32(s_col + c * 32, u);
+#pragma unroll
+        for (int e = 0; e < 32; ++e) s[c * 32 + e] = __uint_as_float(u[e]);
+      }
+      tmem_ld_wait();
+      if (BIAS) {
+#pragma unroll
+        for (int e = 0; e < PA_KEYS; ++e) s[e] = fmaf(s[e], p.scale_log2, tb[-e]);
+      }
+      const bool full = k0 + PA_KEYS - 1 <= pos0[w] && (p.window <= 0 || pos0[w] + n_tok[w] - 1 - k0 < p.window);
+      if (!full) {
+        const int a = first - k0, b = live ? pos - k0 : -1;
+#pragma unroll
+        for (int e = 0; e < PA_KEYS; ++e)
+          if (e < a || e > b) s[e] = -INFINITY;
+      }
+      float mx[4] = {s[0], s[1], s[2], s[3]};
+#pragma unroll
+      for (int e = 4; e < PA_KEYS; ++e) mx[e & 3] = fmaxf(mx[e & 3], s[e]);
+      float top = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
+      if (!BIAS) top *= p.scale_log2;
+      const bool move = top > m + PA_SLACK;
+      if (__any_sync(0xffffffffu, move)) {
+        const float f = move ? pa_ex2(m - top) : 1.0f;
+        if (move) m = top;
+        l *= f;
+        if (n > 0) {                                       // (S(i) follows PV(i - 1) in the pipe: O is at rest)
+#pragma unroll 1
+          for (int c = 0; c < 4; ++c) {
+            uint32_t u[32];
+            tmem_ld_32x32b_x32(o_col + c * 32, u);
+            tmem_ld_wait();
+#pragma unroll
+            for (int e = 0; e < 32; ++e) u[e] = __float_as_uint(__uint_as_float(u[e]) * f);
+            tmem_st_32x32b_x32(o_col + c * 32, u);
+          }
+        }
+      }
+      const float mm = m == -INFINITY ? 0.0f : m;
+      const float2 sc2 = make_float2(p.scale_log2, p.scale_log2), mm2 = make_float2(-mm, -mm);
+      float2 sum[2] = {make_float2(0.0f, 0.0f), make_float2(0.0f, 0.0f)};
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        uint32_t uh[16], ul[16];
+#pragma unroll
+        for (int e = 0; e < 16; ++e) {
+          float2 x = make_float2(s[c * 32 + 2 * e], s[c * 32 + 2 * e + 1]);
+          x = BIAS ? pa_add2(x, mm2) : pa_fma2(x, sc2, mm2);
+          const float2 pe = make_float2(pa_ex2(x.x), pa_ex2(x.y));
+          sum[e & 1] = pa_add2(sum[e & 1], pe);
+          uh[e] = Num<__nv_bfloat16>::pack(pe.x, pe.y);
+          const float2 hf = Num<__nv_bfloat16>::unpack(uh[e]);
+          const float2 lf = pa_fma2(hf, make_float2(-1.0f, -1.0f), pe);
+          ul[e] = Num<__nv_bfloat16>::pack(lf.x, lf.y);
+        }
+        pa_st16(s_col + c * 16, uh);
+        pa_st16(s_col + 64 + c * 16, ul);
+      }
+      l += (sum[0].x + sum[0].y) + (sum[1].x + sum[1].y);
+      tmem_st_wait();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&p_full[w]);
+    }
+    if (n > 0) {
+      guard_wait(&o_full[w], 0, dead);
+      tc_fence_after();
+      float f;
+      if (p.sink) {
+        const float sk = p.sink[live ? h : g * p.per] * PA_LOG2E, M = fmaxf(m, sk), c = pa_ex2(m - M);
+        f = c / (l * c + pa_ex2(sk - M));
+      } else {
+        f = 1.0f / l;
+      }
+      if (*dead) f = NAN;
+      f *= p.out_mul;
+      const int64_t row = q_begin + t0 + w * tpb + tok;
+      __nv_bfloat16* dst = p.out + row * p.out_ts + (int64_t)h * p.out_hs;
+      const __nv_bfloat16* gt = p.gate ? p.gate + row * p.ld_gate + (p.gate_heads ? (int64_t)h : (int64_t)h * PA_VD) : nullptr;
+      if (gt && p.gate_heads && live) f = f / (1.0f + expf(-__bfloat162float(gt[0])));
+      const bool per_channel = gt != nullptr && !p.gate_heads;
+#pragma unroll 1
+      for (int c = 0; c < 4; ++c) {
+        uint32_t u[32];
+        tmem_ld_32x32b_x32(o_col + c * 32, u);
+        tmem_ld_wait();
+        if (live) {
+#pragma unroll
+          for (int e = 0; e < 32; e += 8) {
+            float o[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) o[j] = __uint_as_float(u[e + j]) * f;
+            if (per_channel) {
+              uint32_t gw[4];
+              if (p.gate_vec) {
+                const uint4 t = *reinterpret_cast<const uint4*>(gt + c * 32 + e);
+                gw[0] = t.x; gw[1] = t.y; gw[2] = t.z; gw[3] = t.w;
+              } else {
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                  gw[j] = Num<__nv_bfloat16>::pack(__bfloat162float(gt[c * 32 + e + 2 * j]),
+                                                   __bfloat162float(gt[c * 32 + e + 2 * j + 1]));
+              }
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                const float2 gv = Num<__nv_bfloat16>::unpack(gw[j]);
+                o[2 * j] = o[2 * j] / (1.0f + expf(-gv.x));
+                o[2 * j + 1] = o[2 * j + 1] / (1.0f + expf(-gv.y));
+              }
+            }
+            uint4 v;
+            v.x = Num<__nv_bfloat16>::pack(o[0], o[1]);
+            v.y = Num<__nv_bfloat16>::pack(o[2], o[3]);
+            v.z = Num<__nv_bfloat16>::pack(o[4], o[5]);
+            v.w = Num<__nv_bfloat16>::pack(o[6], o[7]);
+            *reinterpret_cast<uint4*>(dst + c * 32 + e) = v;
+          }
+        }
+      }
+    }
+  }
+  if (threadIdx.x == 8 * 32 && *dead) guard_drain();
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 9) {
+    tc_fence_after();
+    tmem_dealloc(tmem, 512);
+  }
+}
+
+// Paged rows in order; 16-byte pieces.
+__global__ void __launch_bounds__(256)
+prompt_gather_kernel(uint4* __restrict__ dst0, const uint4* __restrict__ src0, int64_t ld0, int vec0,
+                     uint4* __restrict__ dst1, const uint4* __restrict__ src1, int64_t ld1, int vec1,
+                     const int* __restrict__ kv_cu, const int* __restrict__ tables, const int* __restrict__ blk_cu,
+                     int block_size, int rows_per_cta) {
+  const int seq = blockIdx.y, b0 = blk_cu[seq], n_blk = blk_cu[seq + 1] - b0;
+  const int rows = n_blk * block_size + 16, kv_len = kv_cu[seq + 1] - kv_cu[seq];
+  const int64_t out0 = (int64_t)b0 * block_size + 16 * seq;
+  const int per_row = vec0 + vec1;
+  for (int r0 = blockIdx.x * rows_per_cta; r0 < rows; r0 += gridDim.x * rows_per_cta) {
+    const int nr = min(rows_per_cta, rows - r0);
+    for (int e = threadIdx.x; e < nr * per_row; e += 256) {
+      const int rr = e / per_row, c = e - rr * per_row, r = r0 + rr;
+      uint4 v = make_uint4(0u, 0u, 0u, 0u);
+      if (r < kv_len) {
+        const int64_t slot = (int64_t)tables[b0 + r / block_size] + r % block_size;
+        v = c < vec0 ? src0[slot * ld0 + c] : src1[slot * ld1 + (c - vec0)];
+      }
+      if (c < vec0) dst0[(out0 + r) * vec0 + c] = v;
+      else dst1[(out0 + r) * vec1 + (c - vec0)] = v;
+    }
+  }
+}
+
+int encode_rows(CUtensorMap* m, const void* ptr, int64_t cols, int64_t rows, int64_t ld, int box_rows) {
+  tensor_map_encode_fn enc = get_tensor_map_encode();
+  if (!enc) return set_error(B200_ERR_CUDA, "cuTensorMapEncodeTiled entry point unavailable");
+  cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
+  cuuint64_t strides[1] = {(cuuint64_t)ld * 2};
+  cuuint32_t box[2] = {64u, (cuuint32_t)box_rows};
+  cuuint32_t estr[2] = {1, 1};
+  CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), dims, strides, box, estr,
+                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return set_error(B200_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d) for prompt attention", (int)r);
+  return B200_OK;
+}
+
+template <int NA, bool BIAS, typename QT>
+int launch_prompt_attn(const CUtensorMap& kmap, const CUtensorMap& rmap, const CUtensorMap& vmap, const PromptAttnParams& p,
+                       int G, int n_seq, cudaStream_t st) {
+  const size_t smem = 1024 + PaCfg<NA>::TILES + PaCfg<NA>::BARS * 8 + 16 + (BIAS ? 16 * (size_t)p.per * p.tab_ld : 0);
+  B200_CHECK_ARG(smem <= 227 * 1024, "prompt_attn: %d query heads per key head do not fit in shared memory", p.per);
+  auto kern = prompt_attn_kernel<NA, BIAS, QT>;
+  B200_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  kern<<<dim3((unsigned)G, (unsigned)n_seq, (unsigned)p.q_blocks), PA_THREADS, smem, st>>>(kmap, rmap, vmap, p);
+  B200_LAUNCH_OK("prompt_attn_kernel");
+  return B200_OK;
+}
+
+}  // namespace
+}  // namespace b200
+
+using namespace b200;
+
+extern "C" {
+
+int b200_prompt_gather(void* dst0, const void* src0, int64_t ld0, int64_t cols0, void* dst1, const void* src1, int64_t ld1,
+                       int64_t cols1, const int32_t* kv_cu_lens, const int32_t* block_tables, const int32_t* cu_block_lens,
+                       int64_t n_seq, int64_t kv_max, int64_t block_size, b200_stream_t stream) {
+  if (n_seq == 0) return B200_OK;
+  B200_CHECK_ARG(dst0 && src0 && kv_cu_lens && block_tables && cu_block_lens && (!dst1 || src1), "prompt_gather: null pointer");
+  B200_CHECK_ARG(n_seq > 0 && n_seq <= 65535 && kv_max > 0 && block_size > 0 && cols0 > 0 && cols0 % 8 == 0 && ld0 % 8 == 0 &&
+                     ld0 >= cols0 && is_aligned(dst0, 16) && is_aligned(src0, 16) &&
+                     (!dst1 || (cols1 > 0 && cols1 % 8 == 0 && ld1 % 8 == 0 && ld1 >= cols1 && is_aligned(dst1, 16) &&
+                                is_aligned(src1, 16))),
+                 "prompt_gather: rows on 16 bytes");
+  const int vec0 = (int)(cols0 / 8), vec1 = dst1 ? (int)(cols1 / 8) : 0;
+  const int rows_per_cta = 16;
+  const int64_t ctas = (kv_max + block_size + 16 + rows_per_cta - 1) / rows_per_cta;
+  prompt_gather_kernel<<<dim3((unsigned)(ctas < 4096 ? ctas : 4096), (unsigned)n_seq), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+      static_cast<uint4*>(dst0), static_cast<const uint4*>(src0), ld0 / 8, vec0, static_cast<uint4*>(dst1),
+      static_cast<const uint4*>(src1), ld1 / 8, vec1, kv_cu_lens, block_tables, cu_block_lens, (int)block_size, rows_per_cta);
+  B200_LAUNCH_OK("prompt_gather_kernel");
+  return B200_OK;
+}
+
+int b200_prompt_attn(void* out, int64_t out_token_stride, int64_t out_head_stride, const void* q, int64_t q_token_stride,
+                     int64_t q_head_stride, int q_is_fp32, const void* k, int64_t ldk, int64_t k_head_stride,
+                     const void* k_shared, int64_t ld_shared, const void* v, int64_t ldv, int64_t v_head_stride,
+                     int64_t n_key_rows, const float* r1, const float* r2, const float* sink, const void* gate,
+                     int64_t ld_gate, float out_mul, int gate_heads, int64_t window, const int32_t* q_cu_lens,
+                     const int32_t* kv_cu_lens, const int32_t* cu_block_lens, int64_t n_seq, int64_t q_max, int64_t H,
+                     int64_t G, int64_t block_size, float scale, b200_stream_t stream) {
+  if (n_seq == 0 || q_max == 0) return B200_OK;
+  B200_CHECK_ARG(out && q && k && v && q_cu_lens && kv_cu_lens && cu_block_lens && (r1 == nullptr) == (r2 == nullptr),
+                 "prompt_attn: null pointer");
+  B200_CHECK_ARG(n_seq > 0 && n_seq <= 65535 && q_max > 0 && H > 0 && G > 0 && H % G == 0 && 128 % (H / G) == 0 &&
+                     block_size > 0 && scale > 0.0f && window >= 0 && window < (1ll << 30) && n_key_rows > 0 &&
+                     n_key_rows < (1ll << 31) - 256 && (!k_shared || !r1),
+                 "prompt_attn: bad shape (query heads per key head divide 128, a positive scale)");
+  B200_CHECK_ARG(is_aligned(out, 16) && out_token_stride % 8 == 0 && out_head_stride % 8 == 0 && is_aligned(q, 16) &&
+                     q_token_stride % 4 == 0 && q_head_stride % 4 == 0 && is_aligned(k, 16) && ldk % 8 == 0 &&
+                     k_head_stride % 8 == 0 && is_aligned(v, 16) && ldv % 8 == 0 && v_head_stride % 8 == 0 &&
+                     (!k_shared || (is_aligned(k_shared, 16) && ld_shared % 8 == 0)),
+                 "prompt_attn: rows and heads on 16 bytes (queries on 4 channels)");
+  PromptAttnParams p{};
+  p.out = static_cast<__nv_bfloat16*>(out);
+  p.out_ts = out_token_stride; p.out_hs = out_head_stride;
+  p.q = q; p.q_ts = q_token_stride; p.q_hs = q_head_stride;
+  p.q_cu = q_cu_lens; p.kv_cu = kv_cu_lens; p.blk_cu = cu_block_lens;
+  p.r1 = r1; p.r2 = r2; p.sink = sink;
+  p.gate = static_cast<const __nv_bfloat16*>(gate); p.ld_gate = ld_gate;
+  p.gate_heads = gate_heads; p.gate_vec = gate && is_aligned(gate, 16) && ld_gate % 8 == 0;
+  p.out_mul = out_mul; p.scale_log2 = scale * PA_LOG2E;
+  p.block_size = (int)block_size; p.window = (int)window;
+  p.per = (int)(H / G);
+  while ((1 << p.per_log2) < p.per) ++p.per_log2;
+  const int tpb = PA_ROWS / p.per;
+  p.q_blocks = (int)((q_max + 2 * tpb - 1) / (2 * tpb));
+  B200_CHECK_ARG(p.q_blocks <= 65535, "prompt_attn: portion of %lld tokens", (long long)q_max);
+  p.k_hs = (int)k_head_stride; p.v_hs = (int)v_head_stride;
+  // table rows of heads on different banks for the 32 / per tokens a warp reads side by side
+  p.tab_ld = tpb + PA_KEYS - 1;
+  while (p.tab_ld % 32 != (32 / (p.per < 32 ? p.per : 32)) % 32) ++p.tab_ld;
+  CUtensorMap kmap, rmap, vmap;
+  int rc = encode_rows(&kmap, k, (G - 1) * k_head_stride + 128, n_key_rows, ldk, 128);
+  if (rc != B200_OK) return rc;
+  rmap = kmap;
+  if (k_shared) rc = encode_rows(&rmap, k_shared, 64, n_key_rows, ld_shared, 128);
+  if (rc == B200_OK) rc = encode_rows(&vmap, v, (G - 1) * v_head_stride + 128, n_key_rows, ldv, 64);
+  if (rc != B200_OK) return rc;
+  auto st = static_cast<cudaStream_t>(stream);
+#define PA_GO(NA, BIAS)                                                                              \
+  return q_is_fp32 ? launch_prompt_attn<NA, BIAS, float>(kmap, rmap, vmap, p, (int)G, (int)n_seq, st) \
+                   : launch_prompt_attn<NA, BIAS, __nv_bfloat16>(kmap, rmap, vmap, p, (int)G, (int)n_seq, st)
+  if (k_shared) { PA_GO(3, false); }
+  if (r1) { PA_GO(2, true); }
+  PA_GO(2, false);
+#undef PA_GO
+}
+
+int64_t b200_prompt_attn_paged_workspace_bytes(int64_t n_key_rows, int64_t G, int shared_kv) {
+  return n_key_rows * G * 128 * 2 * (shared_kv ? 1 : 2);
+}
+
+int b200_prompt_attn_paged(void* out, int64_t ldo, const void* q, int q_is_fp32, const void* k_cache, const void* v_cache,
+                           void* workspace, int64_t workspace_bytes, int64_t n_key_rows, const float* r1, const float* r2,
+                           const float* sink, const void* gate, int64_t ld_gate, float out_mul, int gate_heads,
+                           int64_t window, const int32_t* q_cu_lens, const int32_t* kv_cu_lens, const int32_t* block_tables,
+                           const int32_t* cu_block_lens, int64_t n_seq, int64_t q_max, int64_t kv_max, int64_t H, int64_t G,
+                           int64_t block_size, float scale, b200_stream_t stream) {
+  if (n_seq == 0 || q_max == 0) return B200_OK;
+  const bool shared = k_cache == v_cache;
+  const int64_t cols = G * 128;
+  B200_CHECK_ARG(workspace && is_aligned(workspace, 16) && G > 0 &&
+                     workspace_bytes >= b200_prompt_attn_paged_workspace_bytes(n_key_rows, G, shared),
+                 "prompt_attn_paged: workspace of %lld key rows required", (long long)n_key_rows);
+  __nv_bfloat16* k = static_cast<__nv_bfloat16*>(workspace);
+  __nv_bfloat16* v = shared ? k : k + n_key_rows * cols;
+  const int rc = b200_prompt_gather(k, k_cache, cols, cols, shared ? nullptr : v, v_cache, cols, cols, kv_cu_lens, block_tables,
+                                    cu_block_lens, n_seq, kv_max, block_size, stream);
+  if (rc != B200_OK) return rc;
+  return b200_prompt_attn(out, ldo, 128, q, H * 128, 128, q_is_fp32, k, cols, 128, nullptr, 0, v, cols, 128, n_key_rows, r1, r2,
+                          sink, gate, ld_gate, out_mul, gate_heads, window, q_cu_lens, kv_cu_lens, cu_block_lens, n_seq, q_max,
+                          H, G, block_size, scale, stream);
+}
+
+}  // extern "C"

@@ -125,7 +125,7 @@ class _Layer:
 @register_model("Gugalorn")
 class GugalornDecoder:
     needs_state_slots = True
-    CSRC = ("postnorm.cu", "hyper.cu", "filters.cu", "linear_scan.cu", "sink_attn.cu")
+    CSRC = ("postnorm.cu", "hyper.cu", "filters.cu", "linear_scan.cu", "sink_attn.cu", "prompt_attn.cu")
 
     def __init__(self, config: dict, dtype: torch.dtype, device, max_seqs: int = 4):
         if dtype not in (torch.bfloat16, torch.float32):

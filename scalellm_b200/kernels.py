@@ -775,6 +775,54 @@ def latent_attn(q_absorbed: torch.Tensor, q: torch.Tensor, cache: torch.Tensor, 
 
 
 # ---------------------------------------------------------------------------
+# prompt portions on the tensor cores over keys and values in order (csrc/prompt_attn.cu)
+# ---------------------------------------------------------------------------
+PROMPT_ATTN_MAX_BYTES = 4 << 30     # of ordered keys and values a call may ask for
+
+
+def prompt_attn_available() -> bool:
+    return _lib.has("b200_prompt_attn")
+
+
+def prompt_key_rows(block_tables: torch.Tensor, block_size: int, n_seq: int) -> int:
+    """Rows of the step's ordered keys: every table entry's block, and the zeros behind every sequence."""
+    return block_tables.numel() * block_size + 16 * n_seq
+
+
+def prompt_gather(caches, kv_cu: torch.Tensor, block_tables: torch.Tensor, cu_block_lens: torch.Tensor, block_size: int,
+                  kv_max: int):
+    """The sequences' rows of one or two caches [slots, ...] (bf16), in order, as [rows, cols] each (see the kernel)."""
+    _cuda(*caches)
+    _check_i32(kv_cu, block_tables, cu_block_lens)
+    n_seq = kv_cu.numel() - 1
+    n = prompt_key_rows(block_tables, block_size, n_seq)
+    src = [c.view(c.shape[0], -1) for c in caches]
+    dst = [torch.empty((n, c.shape[1]), dtype=c.dtype, device=c.device) for c in src]
+    a, b = src[0], src[1] if len(src) > 1 else None
+    check(_lib.load().b200_prompt_gather(_p(dst[0]), _p(a), a.stride(0), a.shape[1], _p(dst[1]) if b is not None else None,
+                                         _p(b), b.stride(0) if b is not None else 0, b.shape[1] if b is not None else 0,
+                                         _p(kv_cu), _p(block_tables), _p(cu_block_lens), n_seq,
+                                         kv_max if kv_max > 0 else n, block_size, _stream()))
+    return dst
+
+
+def prompt_attn(out: torch.Tensor, q: torch.Tensor, k: torch.Tensor, k_head: int, v: torch.Tensor, v_head: int, G: int,
+                q_cu: torch.Tensor, kv_cu: torch.Tensor, cu_block_lens: torch.Tensor, block_size: int, q_max: int,
+                scale: float, window: int = 0, k_shared: Optional[torch.Tensor] = None, r1=None, r2=None, sink=None,
+                gate: Optional[torch.Tensor] = None, gate_heads: int = 0, out_mul: float = 1.0) -> None:
+    """out [rows, H, 128] from q [rows, H, 128 (+ 64)] over ordered keys and values (prompt_gather's rows): k, v [n, ...]
+    with heads k_head / v_head columns apart, k_shared [n, 64] the key channels 128 .. 191 of all heads."""
+    _cuda(out, q, k, v, k_shared, r1, r2, sink, gate)
+    _check_i32(q_cu, kv_cu, cu_block_lens)
+    check(_lib.load().b200_prompt_attn(
+        _p(out), out.stride(0), out.stride(1), _p(q), q.stride(0), q.stride(1), int(q.dtype == torch.float32), _p(k),
+        k.stride(0), k_head, _p(k_shared), k_shared.stride(0) if k_shared is not None else 0, _p(v), v.stride(0), v_head,
+        k.shape[0], _p(r1), _p(r2), _p(sink), _p(gate), gate.stride(0) if gate is not None else 0, out_mul, gate_heads,
+        window, _p(q_cu), _p(kv_cu), _p(cu_block_lens), q_cu.numel() - 1, q_max, q.shape[1], G, block_size, scale,
+        _stream()))
+
+
+# ---------------------------------------------------------------------------
 # generalised delta rule (csrc/delta_rule.cu)
 # ---------------------------------------------------------------------------
 def delta_rule(r: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay_logits: torch.Tensor,
@@ -1349,6 +1397,27 @@ SINK_ATTN_PREFILL_MIN_ROWS = 4
 SINK_ATTN_DECODE_TC_MIN_GROUP = 2
 
 
+# From how many query rows (tokens x query heads per key head) of the longest portion and how many keys a sequence, on
+# average, prompt steps run on csrc/prompt_attn.cu.  Below, a row tile is mostly padding, or the pass that orders the keys
+# is not made up for (16 heads, whole layer on the device: 4 x 128 tokens 46 us against 44 without it, 1 x 64 tokens over
+# 2 112 keys 95 against 170, 16 x 32 over 1 032 keys 74 against 107, 4 x 2 048 tokens 319 against 628).
+SINK_PROMPT_MIN_ROWS = 64
+SINK_PROMPT_MIN_KEYS = 256
+
+
+def _sink_prompt_taken(out, q, k_cache, v_cache, r1, key_rows, scale, n_seq, q_max) -> bool:
+    """Whether the step runs on csrc/prompt_attn.cu: bf16 caches, heads of 128, query heads per key head that divide a
+    tile's 128 rows (at most 8 with a distance bias, whose table per head lies in shared memory), everything on 16 bytes."""
+    per = q.shape[1] // k_cache.shape[1]
+    return (q_max * per >= SINK_PROMPT_MIN_ROWS and key_rows >= SINK_PROMPT_MIN_KEYS * n_seq
+            and k_cache.dtype == torch.bfloat16 and v_cache.dtype == torch.bfloat16
+            and q.shape[2] == 128 and v_cache.shape[2] == 128 and 128 % per == 0 and (r1 is None or per <= 8) and scale > 0
+            and k_cache.is_contiguous() and v_cache.is_contiguous() and q.is_contiguous()
+            and not (out.stride(0) % 8 or out.data_ptr() % 16 or k_cache.data_ptr() % 16 or v_cache.data_ptr() % 16
+                     or q.data_ptr() % 16)
+            and key_rows * k_cache.shape[1] * 512 <= PROMPT_ATTN_MAX_BYTES and prompt_attn_available())
+
+
 def sink_attn(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, r1: Optional[torch.Tensor],
               r2: Optional[torch.Tensor], sink: Optional[torch.Tensor], q_cu: torch.Tensor, kv_cu: torch.Tensor,
               block_tables: torch.Tensor, cu_block_lens: torch.Tensor, token_seq: torch.Tensor, block_size: int,
@@ -1376,6 +1445,16 @@ def sink_attn(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, r1:
     ldo, ldg = out.stride(0), gate.stride(0) if gate is not None else 0
     lib = _lib.load()
     impl = os.environ.get("B200_SINK_ATTN_IMPL")      # "simt": CUDA cores throughout; "simt_decode": for single tokens
+    key_rows = prompt_key_rows(block_tables, block_size, n_seq)
+    if (n_seq > 0 and n_seq == q_cu.numel() - 1 and impl is None
+            and _sink_prompt_taken(out, q, k_cache, v_cache, r1, key_rows, scale, n_seq, q_max)):
+        ws = torch.empty(lib.b200_prompt_attn_paged_workspace_bytes(key_rows, G, v_cache.data_ptr() == k_cache.data_ptr()),
+                         dtype=torch.uint8, device=q.device)
+        check(lib.b200_prompt_attn_paged(_p(out), ldo, _p(q), 1, _p(k_cache), _p(v_cache), _p(ws), ws.numel(), key_rows,
+                                         _p(r1), _p(r2), _p(sink), _p(gate), ldg, out_mul, gate_heads, window, _p(q_cu),
+                                         _p(kv_cu), _p(block_tables), _p(cu_block_lens), n_seq, q_max,
+                                         kv_max if kv_max > 0 else key_rows, H, G, block_size, scale, _stream()))
+        return out
     if (n_seq > 0 and q_max >= SINK_ATTN_PREFILL_MIN_ROWS and impl != "simt"
             and ldo % 2 == 0 and out.data_ptr() % 4 == 0
             and lib.b200_sink_attn_prefill_supported(dim, vdim, _dt(k_cache))):

@@ -131,7 +131,7 @@ class _Layer:
 @register_model("Kigalix")
 class KigalixDecoder:
     needs_state_slots = True
-    CSRC = ("hyper.cu", "latent_attn.cu", "delta_rule.cu", "moe.cu")
+    CSRC = ("hyper.cu", "latent_attn.cu", "prompt_attn.cu", "delta_rule.cu", "moe.cu")
 
     def __init__(self, config: dict, dtype: torch.dtype, device, max_seqs: int = 4):
         if dtype not in (torch.bfloat16, torch.float32):

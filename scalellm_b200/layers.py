@@ -741,6 +741,29 @@ class LatentAttention:
         self.uk = w["uk"].reshape(n_heads, dim, rank).contiguous()               # [H, dim, rank]
         self.uv_t = w["uv"].reshape(n_heads, vdim, rank).transpose(1, 2).contiguous()   # [H, rank, vdim]
         self.o_proj = Linear(w["o"])
+        # prompt steps make keys and values of the cached latents: one product, [key map | value map] head by head
+        self.kv_proj = None
+        if (dim, rot_dim, vdim, dtype) == (128, 64, 128, torch.bfloat16) and rank % 64 == 0 and scale > 0:
+            both = torch.stack([self.uk, w["uv"].reshape(n_heads, vdim, rank)], dim=1)
+            self.kv_proj = Linear(both.reshape(n_heads * (dim + vdim), rank))
+
+    def _makes_keys(self, T: int, params: InputParameters, cache: LatentKVCache) -> bool:
+        """Whether this step makes keys and values of the latents (csrc/prompt_attn.cu) or attends in the latent space.
+        The latter costs 2 (2 rank + rot_dim) FLOPs per (query, key) pair and head, the former 2 (dim + vdim + rot_dim) and
+        a product over all keys of the step's sequences; the rates are what the kernels reach (16 heads, whole layer on the
+        device: 1 x 64 tokens over 2 112 keys 94 us against 134, 16 x 64 over 2 064 250 against 713, 1 x 300 over 4 300 157
+        against 1 096; the 40 us are what 4 x 128 tokens, 107 us, do not make up for)."""
+        if self.kv_proj is None or os.environ.get("B200_LATENT_IMPL") is not None or not kernels.prompt_attn_available():
+            return False
+        n_seq = params.q_cu_seq_lens.numel() - 1
+        keys = kernels.prompt_key_rows(params.block_tables, cache.block_size(), n_seq)
+        if params.q_max_seq_len < 32 or keys * self.H * 512 > kernels.PROMPT_ATTN_MAX_BYTES or cache.rows.stride(0) % 8:
+            return False
+        seen = min(keys / n_seq, self.window + 128.0) if self.window > 0 else keys / n_seq
+        pairs = T * seen * self.H
+        latent = pairs * 2 * (2 * self.rank + self.rd) / 65e12
+        made = 40e-6 + pairs * 2 * (2 * self.dim + self.rd) / 500e12 + keys * self.H * self.rank * 4 * self.dim / 1000e12
+        return made < latent
 
     def forward(self, h: torch.Tensor, positions: torch.Tensor, cache: LatentKVCache,
                 params: InputParameters) -> torch.Tensor:
@@ -750,6 +773,17 @@ class LatentAttention:
         q, dkv = proj[:, : self.q_end], proj[:, self.q_end: self.dkv_end]
         kernels.latent_prepare(q, dkv, cache.rows, self.c_norm, self.inv_freq, self.rot_mult, positions,
                                params.new_cache_slots, H, dim, rd, self.rot_dims, rank, self.eps, self.half_pairs)
+        if self._makes_keys(T, params, cache):
+            c, = kernels.prompt_gather([cache.rows], params.kv_cu_seq_lens, params.block_tables, params.cu_block_lens,
+                                       cache.block_size(), params.kv_max_seq_len)
+            kv = _dense_linear(c[:, :rank], self.kv_proj.weight)
+            o = torch.empty((H, T, self.vd) if self.has_gate else (T, H, self.vd), dtype=h.dtype, device=h.device)
+            kernels.prompt_attn(o.transpose(0, 1) if self.has_gate else o, q.view(T, H, dim + rd), kv, dim + self.vd,
+                                kv[:, dim:], dim + self.vd, H, params.q_cu_seq_lens, params.kv_cu_seq_lens,
+                                params.cu_block_lens, cache.block_size(), params.q_max_seq_len, self.scale, self.window,
+                                c[:, rank:])
+            o = kernels.heads_to_rows(o, proj[:, self.dkv_end:]) if self.has_gate else o.view(T, H * self.vd)
+            return self.o_proj.forward_fusable(o) if self.fusable_out else self.o_proj(o)
         qu = q.view(T, H, dim + rd)[:, :, :dim].transpose(0, 1)                 # [H, T, dim] (strided view)
         qa = torch.bmm(qu, self.uk)                                             # folded query [H, T, rank]
         lat = kernels.latent_attn(qa, q, cache.rows, params.q_cu_seq_lens, params.kv_cu_seq_lens,

@@ -166,7 +166,7 @@ class _Run:
 @register_model("Palulorn")
 class PalulornDecoder:
     needs_state_slots = True
-    CSRC = ("postnorm.cu", "filters.cu", "linear_scan.cu", "mingru.cu", "sink_attn.cu", "moe.cu")
+    CSRC = ("postnorm.cu", "filters.cu", "linear_scan.cu", "mingru.cu", "sink_attn.cu", "prompt_attn.cu", "moe.cu")
 
     def __init__(self, config: dict, dtype: torch.dtype, device, max_seqs: int = 4):
         if dtype not in (torch.bfloat16, torch.float32):

@@ -122,7 +122,7 @@ class _Layer:
 @register_model("Zomurax")
 class ZomuraxDecoder:
     needs_state_slots = False
-    CSRC = ("postnorm.cu", "hyper.cu", "latent_attn.cu", "sink_attn.cu", "moe.cu")
+    CSRC = ("postnorm.cu", "hyper.cu", "latent_attn.cu", "sink_attn.cu", "prompt_attn.cu", "moe.cu")
 
     def __init__(self, config: dict, dtype: torch.dtype, device, max_seqs: int = 4):
         if dtype not in (torch.bfloat16, torch.float32):

@@ -1,0 +1,120 @@
+"""Prompt attention over ordered keys and values (csrc/prompt_attn.cu) against 64-bit softmax attention: ragged portions
+around the edges of row and key tiles, cached prefixes, block sizes, grouped heads, bias, sink, gates and window; rows of
+other sequences and of the cache that nobody holds are infinite and must not be seen."""
+import math
+
+import pytest
+import torch
+
+from scalellm_b200 import kernels
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def paged(lens, bs, width, g):
+    """(cache [slots, width], table, cu_blocks, the rows of every sequence); what no sequence holds is infinite."""
+    nb = [-(-sum(x) // bs) for x in lens]
+    order = torch.randperm(sum(nb) + 3, generator=torch.Generator().manual_seed(1))[: sum(nb)]
+    cu = torch.tensor([0] + list(torch.tensor(nb).cumsum(0)), dtype=torch.int32)
+    cache = torch.full(((sum(nb) + 3) * bs, width), math.inf, dtype=torch.bfloat16, device=DEV)
+    table, rows = (order * bs).to(torch.int32), []
+    for i, x in enumerate(lens):
+        slots = (table[cu[i]: cu[i + 1]].long()[:, None] + torch.arange(bs)).reshape(-1)[: sum(x)].to(DEV)
+        r = torch.randn(sum(x), width, generator=g, device=DEV).to(torch.bfloat16)
+        cache[slots] = r
+        rows.append(r.double())
+    return cache, table.to(DEV), cu.to(DEV), rows
+
+
+def check(out, ref, bound):
+    assert bool(torch.isfinite(out).all())
+    assert bool(((out.double() - ref).abs() <= bound).all()), float(((out.double() - ref).abs() - bound).max())
+
+
+LENS = [[(1, 0)], [(128, 0), (129, 0), (127, 1)], [(300, 100), (5, 260), (64, 64)], [(33, 95), (700, 0)], [(2, 1000), (513, 31)]]
+
+
+@pytest.mark.parametrize("lens", LENS)
+@pytest.mark.parametrize("per,bs,window,bias,sink,gate,q32", [
+    (4, 16, 0, True, True, "", True), (1, 16, 0, False, False, "", False), (2, 8, 130, False, True, "channels", True),
+    (8, 1, 0, True, False, "heads", True), (16, 64, 1, False, False, "", True), (4, 32, 300, True, True, "channels", False)])
+def test_grouped_heads(lens, per, bs, window, bias, sink, gate, q32):
+    G, H, d = 2, 2 * per, 128
+    g = torch.Generator(device=DEV).manual_seed(per * 1000 + bs + len(lens))
+    kc, table, cu, _ = paged(lens, bs, G * d, g)
+    vc = kc.clone()
+    vc[torch.isfinite(kc)] = torch.randn(int(torch.isfinite(kc).sum()), generator=g, device=DEV).to(torch.bfloat16)
+    rows = sum(a for a, _ in lens)
+    cum = lambda v: torch.tensor([0] + list(torch.tensor(v).cumsum(0)), dtype=torch.int32, device=DEV)
+    q_cu, kv_cu = cum([a for a, _ in lens]), cum([a + b for a, b in lens])
+    q = torch.randn(rows, H, d, generator=g, device=DEV).to(torch.bfloat16)
+    q = q.float() if q32 else q
+    u = lambda: 0.05 + 0.5 * torch.rand(H, generator=g, device=DEV)
+    r1, r2 = (u(), u()) if bias else (None, None)
+    sk = torch.randn(H, generator=g, device=DEV) if sink else None
+    gt = {"": None, "channels": torch.randn(rows, H * d + 3, generator=g, device=DEV).to(torch.bfloat16)[:, : H * d],
+          "heads": torch.randn(rows, H, generator=g, device=DEV).to(torch.bfloat16)}[gate]
+    out = torch.full((rows, H, d), 7.0, dtype=torch.bfloat16, device=DEV)
+    k, v = kernels.prompt_gather([kc, vc], kv_cu, table, cu, bs, 0)
+    scale, mul = d ** -0.5, 0.75
+    kernels.prompt_attn(out, q, k, d, v, d, G, q_cu, kv_cu, cu, bs, max(a for a, _ in lens), scale, window, None, r1, r2, sk,
+                        gt, int(gate == "heads"), mul)
+    t0 = 0
+    for i, (a, b) in enumerate(lens):
+        slots = (table[cu[i]: cu[i + 1]].long()[:, None] + torch.arange(bs, device=DEV)).reshape(-1)[: a + b]
+        K, V = kc[slots].double().view(-1, G, d), vc[slots].double().view(-1, G, d)
+        pos, j = torch.arange(b, a + b, device=DEV), torch.arange(a + b, device=DEV)
+        dist = pos[:, None] - j[None, :]
+        ok = (dist >= 0) & (dist < window) if window else dist >= 0
+        for h in range(H):
+            s = q[t0: t0 + a, h].double() @ K[:, h // per].T * scale
+            if bias:
+                s = s - r1[h].double() * torch.log(1.0 + r2[h].double() * dist.clamp(min=0))
+            s = s.masked_fill(~ok, -math.inf)
+            if sink:
+                s = torch.cat([s, sk[h].double().expand(a, 1)], dim=1)
+            p = torch.softmax(s, dim=1)[:, : a + b]
+            ref, mag = p @ V[:, h // per] * mul, p @ V[:, h // per].abs() * mul
+            if gate:
+                sg = torch.sigmoid(gt[t0: t0 + a, h * d: (h + 1) * d].double() if gate == "channels" else
+                                   gt[t0: t0 + a, h: h + 1].double())
+                ref, mag = ref * sg, mag * sg
+            # the result's own rounding (2^-8), and weights off by 2^-16 (two bf16 terms) + fp32 scores of 128 products
+            # (|s| < 64 here: 64 * 128 * 2^-24) relative to the sum of magnitudes
+            check(out[t0: t0 + a, h], ref, 2.0 ** -8 * ref.abs() + (2.0 ** -15 + 2.0 ** -10) * mag + 1e-30)
+        t0 += a
+
+
+@pytest.mark.parametrize("lens", LENS)
+@pytest.mark.parametrize("window", [0, 200])
+def test_shared_key_part(lens, window):
+    H, d, rd, bs = 3, 128, 64, 16
+    g = torch.Generator(device=DEV).manual_seed(len(lens) + window)
+    cache, table, cu, rows_of = paged(lens, bs, 64, g)
+    rows = sum(a for a, _ in lens)
+    cum = lambda v: torch.tensor([0] + list(torch.tensor(v).cumsum(0)), dtype=torch.int32, device=DEV)
+    q_cu, kv_cu = cum([a for a, _ in lens]), cum([a + b for a, b in lens])
+    shared, = kernels.prompt_gather([cache], kv_cu, table, cu, bs, max(a + b for a, b in lens))
+    n = shared.shape[0]
+    kv = torch.randn(n, H * 2 * d, generator=g, device=DEV).to(torch.bfloat16)
+    wide = torch.randn(rows, H * (d + rd) + 8, generator=g, device=DEV).to(torch.bfloat16)
+    q = wide[:, : H * (d + rd)].view(rows, H, d + rd)
+    out = torch.empty((H, rows, d), dtype=torch.bfloat16, device=DEV)
+    kernels.prompt_attn(out.transpose(0, 1), q, kv, 2 * d, kv[:, d:], 2 * d, H, q_cu, kv_cu, cu, bs,
+                        max(a for a, _ in lens), 0.07, window, shared)
+    t0 = 0
+    for i, (a, b) in enumerate(lens):
+        k0 = int(cu[i]) * bs + 16 * i
+        assert torch.equal(shared[k0: k0 + a + b].double(), rows_of[i])
+        assert not bool(shared[k0 + a + b: k0 + (int(cu[i + 1]) - int(cu[i])) * bs + 16].any())
+        pos, j = torch.arange(b, a + b, device=DEV), torch.arange(a + b, device=DEV)
+        dist = pos[:, None] - j[None, :]
+        ok = (dist >= 0) & (dist < window) if window else dist >= 0
+        for h in range(H):
+            kh = torch.cat([kv[k0: k0 + a + b, h * 2 * d: h * 2 * d + d], shared[k0: k0 + a + b]], dim=1).double()
+            V = kv[k0: k0 + a + b, h * 2 * d + d: (h + 1) * 2 * d].double()
+            p = torch.softmax((q[t0: t0 + a, h].double() @ kh.T * 0.07).masked_fill(~ok, -math.inf), dim=1)
+            ref = p @ V
+            check(out[h, t0: t0 + a], ref, 2.0 ** -8 * ref.abs() + (2.0 ** -15 + 2.0 ** -10) * (p @ V.abs()) + 1e-30)
+        t0 += a
