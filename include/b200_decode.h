@@ -861,6 +861,16 @@ B200_API int b200_gated_delta_scan(void* out, int64_t ldo, const float* q, const
                                    const int32_t* positions, const int32_t* state_slots, int64_t n_seq, int64_t H,
                                    int64_t G, int64_t dim, int64_t vdim, float eps, float* raw_workspace /*nullable*/,
                                    int64_t rows, int dtype, b200_stream_t stream);
+/* The same for prompt portions in bf16 with dim = vdim = 128, 16 tokens at a time on the tensor cores (delta_chunk.cu);
+ * q_max: the step's longest portion; out and gate rows on 8 bytes; the workspace (16-byte aligned) holds the read-outs and the
+ * chunks' operands. */
+B200_API int64_t b200_gated_delta_chunked_workspace_bytes(int64_t rows, int64_t n_seq, int64_t H);
+B200_API int b200_gated_delta_chunked(void* out, int64_t ldo, const void* gate_logits, int64_t ld_gate,
+                                      const float* norm_weight, float eps, const float* q, const float* k, const float* v,
+                                      const float* decay, const float* beta, float* state, const int32_t* q_cu_lens,
+                                      const int32_t* positions, const int32_t* state_slots, int64_t n_seq, int64_t rows,
+                                      int64_t q_max, int64_t H, int64_t G, void* workspace, int64_t workspace_bytes,
+                                      b200_stream_t stream);
 /* p = softmax(router_weight h) over E outputs (fp32); choice score c = p + correction (nullable); the outputs form
  * n_groups equal runs of neighbours and only the keep_groups runs with the largest max c can be chosen; the `top`
  * largest c are chosen; weights = chosen p / (their sum + weight_eps).  extra_weight (nullable, fp32 [W]):

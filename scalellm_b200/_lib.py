@@ -187,6 +187,9 @@ SIGNATURES = {
                                         _f32, _int, _vp]),
     "b200_gated_delta_scan": (_int, [_vp, _i64, _vp, _vp, _vp, _vp, _vp, _vp, _i64, _vp, _vp, _vp, _vp, _vp, _i64,
                                      _i64, _i64, _i64, _i64, _f32, _vp, _i64, _int, _vp]),
+    "b200_gated_delta_chunked_workspace_bytes": (_i64, [_i64, _i64, _i64]),
+    "b200_gated_delta_chunked": (_int, [_vp, _i64, _vp, _i64, _vp, _f32, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i64,
+                                        _i64, _i64, _i64, _i64, _vp, _i64, _vp]),
     "b200_moe_route_softmax": (_int, [_vp, _vp, _vp, _vp, _i64, _vp, _vp, _vp, _i64, _i64, _i64, _i64, _i64, _i64,
                                       _f32, _int, _vp]),
     "b200_moe_route_sigmoid": (_int, [_vp, _vp, _vp, _i64, _i64, _i64, _i64, _i64, _i64, _i64, _f32, _f32, _vp]),
@@ -217,7 +220,8 @@ SIGNATURES = {
 # just the sources a model asks for into a library of its own.
 ALL_SOURCES = ("runtime.cu", "elementwise.cu", "sampling.cu", "paged_attn.cu", "prefill_attn.cu", "w4a16.cu",
                "dense.cu", "allreduce.cu", "hyper.cu", "latent_attn.cu", "delta_rule.cu", "moe.cu", "postnorm.cu", "mingru.cu",
-               "diff_attn.cu", "sink_attn.cu", "sigmoid_attn.cu", "filters.cu", "linear_scan.cu", "prompt_attn.cu")
+               "diff_attn.cu", "sink_attn.cu", "sigmoid_attn.cu", "filters.cu", "linear_scan.cu", "prompt_attn.cu",
+               "delta_chunk.cu")
 
 _lib: Optional[C.CDLL] = None
 _lib_sources: frozenset = frozenset()

@@ -170,7 +170,7 @@ class _Layer:
 @register_model("Fesupel")
 class FesupelDecoder:
     needs_state_slots = True
-    CSRC = ("postnorm.cu", "hyper.cu", "sigmoid_attn.cu", "delta_rule.cu", "moe.cu")
+    CSRC = ("postnorm.cu", "hyper.cu", "sigmoid_attn.cu", "delta_rule.cu", "delta_chunk.cu", "moe.cu")
 
     def __init__(self, config: dict, dtype: torch.dtype, device, max_seqs: int = 4):
         if dtype not in (torch.bfloat16, torch.float32):

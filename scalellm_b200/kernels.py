@@ -1606,6 +1606,8 @@ def gated_delta_prepare(q_in: torch.Tensor, k_in: torch.Tensor, v_in: torch.Tens
 
 # a step whose longest portion has at least this many tokens norms and gates the read-outs in a launch of its own
 GATED_DELTA_SPLIT_NORM_MIN_ROWS = 16
+# ... and from here on, in bf16 with heads of 128 x 128, runs 16 tokens at a time on the tensor cores (csrc/delta_chunk.cu)
+GATED_DELTA_CHUNK_MIN_ROWS = 16
 
 
 def gated_delta_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.Tensor, beta: torch.Tensor,
@@ -1625,6 +1627,15 @@ def gated_delta_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: t
     assert gate_logits.shape == (rows, H * vdim) and gate_logits.stride(1) == 1
     assert norm_weight.numel() == vdim and state.shape[1:] == (H, dim, vdim)
     out = torch.empty((rows, H * vdim), dtype=gate_logits.dtype, device=q.device)
+    if (q_max >= GATED_DELTA_CHUNK_MIN_ROWS and gate_logits.dtype == torch.bfloat16 and dim == 128 and vdim == 128
+            and gate_logits.stride(0) % 4 == 0 and gate_logits.data_ptr() % 8 == 0 and _lib.has("b200_gated_delta_chunked")):
+        n_seq = state_slots.numel()
+        ws = torch.empty(_lib.load().b200_gated_delta_chunked_workspace_bytes(rows, n_seq, H), dtype=torch.uint8, device=q.device)
+        check(_lib.load().b200_gated_delta_chunked(_p(out), H * vdim, _p(gate_logits), gate_logits.stride(0), _p(norm_weight),
+                                                   eps, _p(q), _p(k), _p(v), _p(decay), _p(beta), _p(state), _p(q_cu),
+                                                   _p(positions), _p(state_slots), n_seq, rows, q_max, H, G, _p(ws),
+                                                   ws.numel(), _stream()))
+        return out
     raw = None
     if q_max >= GATED_DELTA_SPLIT_NORM_MIN_ROWS:
         raw = torch.empty((rows, H * vdim), dtype=torch.float32, device=q.device)

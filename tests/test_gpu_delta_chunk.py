@@ -1,0 +1,50 @@
+"""The gated delta rule over prompt portions, 16 tokens at a time (csrc/delta_chunk.cu), against the recurrence in 64 bits:
+lengths around a chunk, fresh and carried states, weak and very strong decays, strided gates, few and many CTAs."""
+import pytest
+import torch
+
+from scalellm_b200 import kernels
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("lens,H,G,strength", [([16], 2, 1, 0.1), ([17, 33, 1, 5, 2], 4, 2, 0.1), ([100, 300], 4, 4, 1.0),
+                                                ([64, 40], 2, 1, 60.0), ([31, 32, 48], 16, 8, 0.02), ([40] * 10, 8, 4, 2.0)])
+def test_against_64_bits(lens, H, G, strength, monkeypatch):
+    d, rows, n_seq = 128, sum(lens), len(lens)
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    r = lambda *s: torch.randn(s, generator=g, device="cuda")
+    unit = lambda x: x / x.norm(dim=-1, keepdim=True)
+    q, k, v = unit(r(rows, G, d)) * d ** -0.5, unit(r(rows, G, d) + 0.3), r(rows, H, d)
+    decay = torch.exp(-strength * torch.rand(rows, H, d, generator=g, device="cuda") ** 4)
+    beta = torch.rand(rows, H, generator=g, device="cuda")
+    gate = r(rows, H * d + 4).to(torch.bfloat16)[:, : H * d]
+    nw = 1.0 + 0.2 * r(d)
+    q_cu = torch.tensor([0] + list(torch.tensor(lens).cumsum(0)), dtype=torch.int32, device="cuda")
+    pos = torch.cat([torch.arange(n) + (0 if i % 2 == 0 else 7) for i, n in enumerate(lens)]).to(torch.int32).cuda()
+    slots = torch.randperm(n_seq + 2, generator=torch.Generator().manual_seed(1))[: n_seq].to(torch.int32).cuda()
+    state = r(n_seq + 2, H, d, d)
+    before = state.clone()
+    launches = kernels.launch_count()
+    out = kernels.gated_delta_scan(q, k, v, decay, beta, gate, nw, state, q_cu, pos, slots, 1e-5, max(lens))
+    assert kernels.launch_count() - launches == 3                       # chunks, scan, norm and gate
+    ref = torch.zeros(rows, H, d, dtype=torch.float64, device="cuda")
+    want = before.double()
+    for i, n in enumerate(lens):
+        S = torch.zeros(H, d, d, dtype=torch.float64, device="cuda") if i % 2 == 0 else before[slots[i].long()].double()
+        for t in range(int(q_cu[i]), int(q_cu[i]) + n):
+            kk, qq = (x[t].double().repeat_interleave(H // G, 0) for x in (k, q))
+            S = S * decay[t].double()[:, :, None]
+            u = beta[t].double()[:, None] * (v[t].double() - torch.einsum("hkv,hk->hv", S, kk))
+            S = S + kk[:, :, None] * u[:, None, :]
+            ref[t] = torch.einsum("hkv,hk->hv", S, qq)
+        want[slots[i].long()] = S
+    # operands of two bf16 terms are off by 2^-17 of their size; a state is a sum of about 16 to 1 000 updates whose errors
+    # do not line up: 2^-14 of the state's norm bounds them per head
+    err = (state.double() - want).flatten(2).norm(dim=2)
+    assert bool((err <= 2.0 ** -14 * want.flatten(2).norm(dim=2) + 1e-30).all())
+    inv = 1.0 / torch.sqrt((ref * ref).mean(dim=-1, keepdim=True) + 1e-5)
+    full = ref * inv * nw.double() * torch.sigmoid(gate.double().view(rows, H, d))
+    # the result's rounding (2^-8 of the value) and the same relative error against the row
+    bound = 2.0 ** -8 * full.abs() + 2.0 ** -12 * (inv * ref.norm(dim=-1, keepdim=True)) * nw.double().abs()
+    assert bool(((out.double().view(rows, H, d) - full).abs() <= bound).all())
