@@ -20,33 +20,58 @@ constexpr int kMaxExperts = 1024;
 constexpr int kMaxTop = 32;
 constexpr int BM = 64, BN = 64, BK = 16;
 
-template <typename T>
-__global__ void __launch_bounds__(128)
+// A CTA per row, a warp per expert in turn.  Four values a lane and load where rows allow it (VEC): a decode step's few
+// rows are bound by the latency of their loads, so they are few and all in flight (16 rows, 8 experts, W 2048: 16 -> 8 us).
+constexpr int RT_WARPS = 8;
+template <typename T, bool VEC>
+__global__ void __launch_bounds__(RT_WARPS * 32)
 moe_route_kernel(int* __restrict__ ids, float* __restrict__ weights, const T* __restrict__ h, int64_t ldh,
                  const float* __restrict__ Wr, int W, int E, int top) {
   __shared__ float z_s[kMaxExperts];
   const int row = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const T* x = h + (size_t)row * ldh;
-  for (int e = warp; e < E; e += 4) {
+  for (int e = warp; e < E; e += RT_WARPS) {
     const float* w = Wr + (size_t)e * W;
     float acc = 0.0f;
-    for (int i = lane; i < W; i += 32) acc += Num<T>::to_f(x[i]) * w[i];
+    if (VEC) {
+      float part[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll 8
+      for (int i = lane * 4; i < W; i += 128) {
+        float xv[4], wv[4];
+        load4<T>(x + i, xv);
+        load4<float>(w + i, wv);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) part[j] += xv[j] * wv[j];
+      }
+      acc = (part[0] + part[1]) + (part[2] + part[3]);
+    } else {
+      for (int i = lane; i < W; i += 32) acc += Num<T>::to_f(x[i]) * w[i];
+    }
     acc = warp_sum(acc);
     if (lane == 0) z_s[e] = acc;
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int k = 0; k < top; ++k) {
-      int best = 0;
-      float bz = -INFINITY;
-      for (int e = 0; e < E; ++e) {
-        const float z = z_s[e];
-        if (z > bz) { bz = z; best = e; }
-      }
+  if (warp != 0) return;
+  for (int k = 0; k < top; ++k) {                            // the largest logit; the first of equal ones
+    int best = E;
+    float bz = -INFINITY;
+    for (int e = lane; e < E; e += 32) {
+      const float z = z_s[e];
+      if (z > bz) { bz = z; best = e; }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const float oz = __shfl_xor_sync(0xffffffffu, bz, o);
+      const int ob = __shfl_xor_sync(0xffffffffu, best, o);
+      if (oz > bz || (oz == bz && ob < best)) { bz = oz; best = ob; }
+    }
+    if (best == E) best = 0;                                 // (nothing above -inf is left)
+    if (lane == 0) {
       ids[(size_t)row * top + k] = best;
       weights[(size_t)row * top + k] = 1.0f / (1.0f + expf(-bz));
       z_s[best] = -INFINITY;
     }
+    __syncwarp();
   }
 }
 
@@ -357,18 +382,44 @@ __global__ void moe_gather_kernel(T* __restrict__ xs, const T* __restrict__ h, i
 }
 
 // out[row] = scale * sum_k Y[pos_of_pair[row, k]] (+ addend[row]: a result every token gets, a shared expert's)
-template <typename T>
-__global__ void moe_combine_kernel(T* __restrict__ out, const T* __restrict__ Y, int64_t ldy,
-                                   const int* __restrict__ pos_of_pair, int W, int top, float scale,
-                                   const T* __restrict__ addend, int64_t ld_add) {
+// V values a thread: 16 bytes where the rows allow it, all of a row's loads in flight (16 rows of 2048: 14 -> 4 us).
+template <typename T, int V>
+__global__ void __launch_bounds__(256)
+moe_combine_kernel(T* __restrict__ out, const T* __restrict__ Y, int64_t ldy, const int* __restrict__ pos_of_pair, int W,
+                   int top, float scale, const T* __restrict__ addend, int64_t ld_add) {
   const int row = blockIdx.x;
-  for (int i = threadIdx.x; i < W; i += blockDim.x) {
-    float acc = 0.0f;
-    for (int k = 0; k < top; ++k)
-      acc += Num<T>::to_f(Y[(size_t)pos_of_pair[(size_t)row * top + k] * ldy + i]);
-    acc *= scale;
-    if (addend) acc += Num<T>::to_f(addend[(size_t)row * ld_add + i]);
-    out[(size_t)row * W + i] = Num<T>::from_f(acc);
+  const int* pos = pos_of_pair + (size_t)row * top;
+  for (int i = (blockIdx.y * 256 + threadIdx.x) * V; i < W; i += gridDim.y * 256 * V) {
+    float acc[V];
+#pragma unroll
+    for (int j = 0; j < V; ++j) acc[j] = 0.0f;
+    auto add = [&](const T* src) {
+      if constexpr (V == 1) {
+        acc[0] += Num<T>::to_f(src[0]);
+      } else {
+#pragma unroll
+        for (int j = 0; j < V; j += 4) {
+          float v[4];
+          load4<T>(src + j, v);
+#pragma unroll
+          for (int q = 0; q < 4; ++q) acc[j + q] += v[q];
+        }
+      }
+    };
+#pragma unroll 4
+    for (int k = 0; k < top; ++k) add(Y + (size_t)pos[k] * ldy + i);
+#pragma unroll
+    for (int j = 0; j < V; ++j) acc[j] *= scale;
+    if (addend) add(addend + (size_t)row * ld_add + i);
+    T* o = out + (size_t)row * W + i;
+    if constexpr (V == 1) {
+      o[0] = Num<T>::from_f(acc[0]);
+    } else {
+      T t[V];
+#pragma unroll
+      for (int j = 0; j < V; ++j) t[j] = Num<T>::from_f(acc[j]);
+      *reinterpret_cast<uint4*>(o) = *reinterpret_cast<const uint4*>(t);
+    }
   }
 }
 
@@ -633,9 +684,10 @@ int b200_moe_route(int32_t* expert_ids, float* weights, const void* h, int64_t l
                      top <= kMaxTop,
                  "moe_route: bad shape (experts <= 1024, top <= min(experts, 32))");
   auto st = static_cast<cudaStream_t>(stream);
-  MOE_DISPATCH(dtype, (moe_route_kernel<T><<<(unsigned)rows, 128, 0, st>>>(
-                          expert_ids, weights, static_cast<const T*>(h), ldh, router_weight, (int)W, (int)E,
-                          (int)top)));
+  const int es = dtype == B200_FP32 ? 4 : 2;
+  const bool vec = W % 4 == 0 && ldh % 4 == 0 && is_aligned(h, 4 * es) && is_aligned(router_weight, 16);
+  MOE_DISPATCH(dtype, (vec ? moe_route_kernel<T, true> : moe_route_kernel<T, false>)<<<(unsigned)rows, RT_WARPS * 32, 0, st>>>(
+                          expert_ids, weights, static_cast<const T*>(h), ldh, router_weight, (int)W, (int)E, (int)top));
   B200_LAUNCH_OK("moe_route_kernel");
   return B200_OK;
 }
@@ -731,9 +783,14 @@ int b200_moe_combine(void* out, const void* Y, int64_t ldy, const int32_t* pos_o
   B200_CHECK_ARG(out && Y && pos_of_pair, "moe_combine: null pointer");
   B200_CHECK_ARG(rows > 0 && W > 0 && ldy >= W && top >= 1 && (!addend || ld_add >= W), "moe_combine: bad shape");
   auto st = static_cast<cudaStream_t>(stream);
-  MOE_DISPATCH(dtype, (moe_combine_kernel<T><<<(unsigned)rows, 128, 0, st>>>(
+  const int es = dtype == B200_FP32 ? 4 : 2, per16 = 16 / es;
+  const bool vec = W % per16 == 0 && ldy % per16 == 0 && is_aligned(out, 16) && is_aligned(Y, 16) &&
+                   (!addend || (ld_add % per16 == 0 && is_aligned(addend, 16)));
+  const int64_t per_cta = 256 * (vec ? per16 : 1);
+  const dim3 grid((unsigned)rows, (unsigned)(rows >= 1024 ? 1 : (W + per_cta - 1) / per_cta < 16 ? (W + per_cta - 1) / per_cta : 16));
+  MOE_DISPATCH(dtype, (vec ? moe_combine_kernel<T, 16 / sizeof(T)> : moe_combine_kernel<T, 1>)<<<grid, 256, 0, st>>>(
                           static_cast<T*>(out), static_cast<const T*>(Y), ldy, pos_of_pair, (int)W, (int)top, scale,
-                          static_cast<const T*>(addend), ld_add)));
+                          static_cast<const T*>(addend), ld_add));
   B200_LAUNCH_OK("moe_combine_kernel");
   return B200_OK;
 }
