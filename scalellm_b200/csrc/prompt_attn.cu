@@ -13,7 +13,8 @@
 //   attend  : one CTA per (sequence, key/value head, 2 x 128 query rows); a tile's rows are its tokens x the query heads
 //             of the key/value head.  Key tiles of 128.
 //
-// Warps 0-3 and 4-7 are two softmax groups, one per 128-row tile, a thread per row; warp 8 loads, warp 9 issues MMAs:
+// Warps 0-7 and 8-15 are two softmax groups, one per 128-row tile, two threads per row (64 keys of the tile each: one
+// warp a scheduler and tile is bound by its own instruction latency); warp 16 loads, warp 17 issues MMAs:
 //   S_w = Q_w K^T -> TMEM;  softmax group w turns S_w into weights IN PLACE, as two bf16 terms per weight (high and low
 //   part: 16 bits of mantissa, exactly the 128 fp32 columns' space);  O_w += P_hi V + P_lo V with P read from TMEM.
 // While one group works on its scores the tensor pipe runs the other tile's products (PV_0 S_0' PV_1 S_1' ...).  The
@@ -21,8 +22,9 @@
 // 2^8; its rounding is relative all the same), so O is almost never rescaled: it stays in TMEM until the end.
 //
 // Bound by the chain scores -> weights -> products of a tile: per 128 x 128 tile 2 x (64 NA + 256) x 128 x 128 FLOPs, where
-// the low parts are a third.  4 prompts of up to 2 048 tokens, 16 heads: 160 us with 192-wide keys (the kernel that attends in
-// the latent space: 3.9 ms), 138 us with bias and sink over 4 key heads (mma.sync kernel: 430 us).
+// the low parts are a third; the score products read both operands from shared memory at its full rate.  4 prompts of up to
+// 2 048 tokens, 16 heads: 146 us with 192-wide keys (160 with a thread per row; the kernel that attends in the latent space:
+// 3.9 ms), 138 us with bias and sink over 4 key heads (mma.sync kernel: 430 us).
 #include "common.cuh"
 #include "guard.cuh"
 
@@ -32,7 +34,8 @@ namespace {
 constexpr int PA_ROWS = 128, PA_KEYS = 128, PA_VD = 128;
 constexpr int PA_ATOM = 128 * 128;              // [128 rows x 64] bf16, 128-byte swizzle
 constexpr int PA_VHALF = 64 * 128 * 2;          // V of 64 keys: two [64 keys x 64] chunks
-constexpr int PA_THREADS = 12 * 32;             // two softmax warpgroups; loads, MMAs and two idle warps
+constexpr int PA_SOFT = 16;                     // softmax warps: eight a row tile, two threads a row
+constexpr int PA_THREADS = (PA_SOFT + 4) * 32;  // and a warpgroup: one warp loads, one issues MMAs, two idle
 constexpr float PA_LOG2E = 1.4426950408889634f;
 constexpr float PA_SLACK = 8.0f;                // log2 of the growth of a row's maximum that is tolerated
 
@@ -98,7 +101,8 @@ __global__ void __launch_bounds__(PA_THREADS, 1)
 prompt_attn_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__ CUtensorMap rmap,
                    const __grid_constant__ CUtensorMap vmap, const PromptAttnParams p) {
   using Cfg = PaCfg<NA>;
-  extern __shared__ uint8_t smem_dyn[];
+  extern __shared__ __align__(1024) uint8_t smem_dyn[];
+  if (smem_u32(smem_dyn) & 1023u) return;                  // (the tiles' swizzle counts on it; the declaration gives it)
   const int g = blockIdx.x, seq = blockIdx.y, qb = p.q_blocks - 1 - (int)blockIdx.z;   // long walks first
   const int tpb = PA_ROWS >> p.per_log2;
   const int q_begin = p.q_cu[seq], q_len = p.q_cu[seq + 1] - q_begin;
@@ -118,7 +122,7 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_consta
   }
   const int i0 = lo[0], i1 = max(hi[0], hi[1]);            // (tile 1 starts no earlier than tile 0 and ends no earlier)
 
-  uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~static_cast<uintptr_t>(1023));
+  uint8_t* base = smem_dyn;
   uint8_t* q_smem = base;                                  // [2][NA] atoms
   uint8_t* k_smem = q_smem + 2 * NA * PA_ATOM;             // [KST][NA] atoms
   uint8_t* v_smem = k_smem + Cfg::KST * NA * PA_ATOM;      // [NV] halves
@@ -133,22 +137,23 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_consta
   uint64_t* o_full = p_full + 2;                           // [2]
   uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(bars + Cfg::BARS);
   volatile uint32_t* dead = tmem_holder + 1;
-  float* tab = reinterpret_cast<float*>(tmem_holder + 4);  // [2 groups][2][per][tab_ld] (distance bias)
+  float* xch = reinterpret_cast<float*>(tmem_holder + 4);  // [2 tiles][2 halves][128 rows]: maxima, then sums, crossing
+  float* tab = xch + 2 * 2 * PA_ROWS;                      // [2 tiles][2][per][tab_ld] (distance bias)
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
-    mbar_init(q_full, 8);
+    mbar_init(q_full, PA_SOFT);
     for (int i = 0; i < Cfg::KST; ++i) { mbar_init(&k_full[i], 1); mbar_init(&k_empty[i], 1); }
     for (int i = 0; i < Cfg::NV; ++i) { mbar_init(&v_full[i], 1); mbar_init(&v_empty[i], 1); }
-    for (int i = 0; i < 2; ++i) { mbar_init(&s_full[i], 1); mbar_init(&p_full[i], 4); mbar_init(&o_full[i], 1); }
+    for (int i = 0; i < 2; ++i) { mbar_init(&s_full[i], 1); mbar_init(&p_full[i], PA_SOFT / 2); mbar_init(&o_full[i], 1); }
     *dead = 0u;
     fence_mbar_init();
   }
-  if (warp == 9) {
+  if (warp == PA_SOFT + 1) {
     tmem_alloc(tmem_holder, 512);
     tmem_relinquish();
   }
-  if (warp == 8 && lane == 0) {
+  if (warp == PA_SOFT && lane == 0) {
     prefetch_tensormap(&kmap);
     if (NA == 3) prefetch_tensormap(&rmap);
     prefetch_tensormap(&vmap);
@@ -158,10 +163,10 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_consta
   tc_fence_after();
   const uint32_t tmem = *tmem_holder;                      // S_0 | S_1 | O_0 | O_1, 128 columns each
 
-  // 384 threads x 168 registers at launch = 256 x 200 + 128 x 104: a softmax thread holds its row's 128 scores
-  if (warp >= 8) {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 104;");
-    if (warp == 8) {
+  // 640 threads x 96 registers at launch = 512 x 104 + 128 x 64
+  if (warp >= PA_SOFT) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
+    if (warp == PA_SOFT) {
       if (lane == 0) {
         for (int i = i0; i < i1; ++i) {
           const int n = i - i0, s = n % Cfg::KST, row = key0 + i * PA_KEYS;
@@ -183,7 +188,7 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_consta
         }
       }
       __syncwarp();
-    } else if (warp == 9) {
+    } else if (warp == PA_SOFT + 1) {
       // (the whole warp walks the loop and one elected lane issues: descriptors stay in uniform registers)
       const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
       const uint64_t qd = umma_desc_kmajor_sw128(__shfl_sync(0xffffffffu, smem_u32(q_smem), 0));
@@ -191,7 +196,8 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_consta
       const uint64_t vd = pa_desc_v(__shfl_sync(0xffffffffu, smem_u32(v_smem), 0));
       auto in_range = [&](int w, int i) { return i >= lo[w] && i < hi[w]; };
       auto scores = [&](int w, int i) {
-        const uint64_t a = qd + w * (NA * PA_ATOM >> 4), b = kd + ((i - i0) % Cfg::KST) * (NA * PA_ATOM >> 4);
+        uint64_t a = qd + w * (NA * PA_ATOM >> 4), b = kd + ((i - i0) % Cfg::KST) * (NA * PA_ATOM >> 4);
+        asm volatile("" : "+l"(a), "+l"(b));               // (the offsets are added where they are used: few registers)
         if (elect_one()) {
 #pragma unroll
           for (int ks = 0; ks < NA * 4; ++ks) {
@@ -236,7 +242,8 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_consta
                 guard_wait(&v_full[sv], (nv / Cfg::NV) & 1, dead);
                 tc_fence_after();
               }
-              const uint64_t v = vd + sv * (PA_VHALF >> 4);
+              uint64_t v = vd + sv * (PA_VHALF >> 4);
+            asm volatile("" : "+l"(v));
               const uint32_t acc = done[w] > 0 || half > 0 ? 1u : 0u;
               const int n_steps = steps - half * 4;
               if (elect_one()) {
@@ -263,21 +270,21 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_consta
       }
     }
   } else {
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 200;");
-    const int w = warp >> 2, r = threadIdx.x & 127;        // this thread's row of tile w
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 104;");
+    const int w = warp >> 3, hf = (warp >> 2) & 1, r = threadIdx.x & 127;   // row r of tile w, its keys and channels 64 hf ..
     const int tok = r >> p.per_log2, hh = r & (p.per - 1), h = g * p.per + hh;
     const bool live = tok < n_tok[w];
     const uint32_t lane_off = (uint32_t)((warp & 3) * 32) << 16;
-    // Q: a warp stages its 32 rows, 4 channels a lane, as the K-major swizzled operand
+    // Q: a warp stages 16 rows, 4 channels a lane, as the K-major swizzled operand
     {
       uint8_t* qt = q_smem + w * NA * PA_ATOM;
-      constexpr int PER = (NA * 64 + 127) / 128, BATCH = 16;   // pieces of a row a lane loads; rows in flight
+      constexpr int PER = (NA * 64 + 127) / 128, BATCH = 8;   // pieces of a row a lane loads; rows in flight
 #pragma unroll 1
-      for (int j0 = 0; j0 < 32; j0 += BATCH) {
+      for (int j0 = 0; j0 < 16; j0 += BATCH) {
         float v[BATCH][PER][4];
 #pragma unroll
         for (int j = 0; j < BATCH; ++j) {
-          const int rr = (warp & 3) * 32 + j0 + j, tk = rr >> p.per_log2, hq = g * p.per + (rr & (p.per - 1));
+          const int rr = (warp & 7) * 16 + j0 + j, tk = rr >> p.per_log2, hq = g * p.per + (rr & (p.per - 1));
           const QT* src = static_cast<const QT*>(p.q) + (int64_t)(q_begin + t0 + w * tpb + tk) * p.q_ts + (int64_t)hq * p.q_hs;
 #pragma unroll
           for (int c = 0; c < PER; ++c) {
@@ -288,7 +295,7 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_consta
         }
 #pragma unroll
         for (int j = 0; j < BATCH; ++j) {
-          const int rr = (warp & 3) * 32 + j0 + j;
+          const int rr = (warp & 7) * 16 + j0 + j;
 #pragma unroll
           for (int c = 0; c < PER; ++c) {
             const int d = lane * 4 + c * 128;
@@ -317,41 +324,49 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_consta
       if (BIAS) {
         float* t = tab + (w * 2 + (n & 1)) * p.per * p.tab_ld;
         const int d0 = pos0[w] - k0 - (PA_KEYS - 1);       // distance of table entry 0
-        for (int e = r; e < p.per * p.tab_ld; e += 128) {
+        for (int e = r + 128 * hf; e < p.per * p.tab_ld; e += 256) {
           const int eh = e / p.tab_ld, ed = e - eh * p.tab_ld;
           const float b1 = p.r1[g * p.per + eh], b2 = p.r2[g * p.per + eh];
           t[e] = -b1 * PA_LOG2E * logf(1.0f + b2 * (float)(d0 + ed));
         }
-        asm volatile("bar.sync %0, 128;" ::"r"(1 + w) : "memory");
-        tb = t + hh * p.tab_ld + tok + PA_KEYS - 1;        // tb[-e]: the bias of key k0 + e
+        asm volatile("bar.sync %0, 256;" ::"r"(1 + w) : "memory");
+        tb = t + hh * p.tab_ld + tok + PA_KEYS - 1 - 64 * hf;              // tb[-e]: the bias of this thread's key e
       }
       guard_wait(&s_full[w], n & 1, dead);
       tc_fence_after();
-      float s[PA_KEYS];
+      float s[64];
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
+      for (int c = 0; c < 2; ++c) {
         uint32_t u[32];
-        tmem_ld_32x32b_x32(s_col + c * 32, u);
+        tmem_ld_32x32b_x32(s_col + hf * 64 + c * 32, u);
 #pragma unroll
         for (int e = 0; e < 32; ++e) s[c * 32 + e] = __uint_as_float(u[e]);
       }
       tmem_ld_wait();
       if (BIAS) {
 #pragma unroll
-        for (int e = 0; e < PA_KEYS; ++e) s[e] = fmaf(s[e], p.scale_log2, tb[-e]);
+        for (int e = 0; e < 64; ++e) s[e] = fmaf(s[e], p.scale_log2, tb[-e]);
       }
       const bool full = k0 + PA_KEYS - 1 <= pos0[w] && (p.window <= 0 || pos0[w] + n_tok[w] - 1 - k0 < p.window);
       if (!full) {
-        const int a = first - k0, b = live ? pos - k0 : -1;
+        const int a = first - k0 - 64 * hf, b = live ? pos - k0 - 64 * hf : -1;
 #pragma unroll
-        for (int e = 0; e < PA_KEYS; ++e)
+        for (int e = 0; e < 64; ++e)
           if (e < a || e > b) s[e] = -INFINITY;
       }
       float mx[4] = {s[0], s[1], s[2], s[3]};
 #pragma unroll
-      for (int e = 4; e < PA_KEYS; ++e) mx[e & 3] = fmaxf(mx[e & 3], s[e]);
+      for (int e = 4; e < 64; ++e) mx[e & 3] = fmaxf(mx[e & 3], s[e]);
       float top = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
       if (!BIAS) top *= p.scale_log2;
+      {
+        // the row's maximum crosses between its two threads; past the barrier both have read their scores, whose columns
+        // the weights go to.  (Written again only after S(i + 1), which follows both threads' weights of this tile.)
+        float* x = xch + w * 2 * PA_ROWS + r;
+        x[hf * PA_ROWS] = top;
+        asm volatile("bar.sync %0, 256;" ::"r"(3 + w) : "memory");
+        top = fmaxf(top, x[(hf ^ 1) * PA_ROWS]);
+      }
       const bool move = top > m + PA_SLACK;
       if (__any_sync(0xffffffffu, move)) {
         const float f = move ? pa_ex2(m - top) : 1.0f;
@@ -359,7 +374,7 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_consta
         l *= f;
         if (n > 0) {                                       // (S(i) follows PV(i - 1) in the pipe: O is at rest)
 #pragma unroll 1
-          for (int c = 0; c < 4; ++c) {
+          for (int c = 2 * hf; c < 2 * hf + 2; ++c) {
             uint32_t u[32];
             tmem_ld_32x32b_x32(o_col + c * 32, u);
             tmem_ld_wait();
@@ -373,7 +388,7 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_consta
       const float2 sc2 = make_float2(p.scale_log2, p.scale_log2), mm2 = make_float2(-mm, -mm);
       float2 sum[2] = {make_float2(0.0f, 0.0f), make_float2(0.0f, 0.0f)};
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
+      for (int c = 0; c < 2; ++c) {
         uint32_t uh[16], ul[16];
 #pragma unroll
         for (int e = 0; e < 16; ++e) {
@@ -382,12 +397,12 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_consta
           const float2 pe = make_float2(pa_ex2(x.x), pa_ex2(x.y));
           sum[e & 1] = pa_add2(sum[e & 1], pe);
           uh[e] = Num<__nv_bfloat16>::pack(pe.x, pe.y);
-          const float2 hf = Num<__nv_bfloat16>::unpack(uh[e]);
-          const float2 lf = pa_fma2(hf, make_float2(-1.0f, -1.0f), pe);
-          ul[e] = Num<__nv_bfloat16>::pack(lf.x, lf.y);
+          const float2 hi2 = Num<__nv_bfloat16>::unpack(uh[e]);
+          const float2 lo2 = pa_fma2(hi2, make_float2(-1.0f, -1.0f), pe);
+          ul[e] = Num<__nv_bfloat16>::pack(lo2.x, lo2.y);
         }
-        pa_st16(s_col + c * 16, uh);
-        pa_st16(s_col + 64 + c * 16, ul);
+        pa_st16(s_col + hf * 32 + c * 16, uh);
+        pa_st16(s_col + 64 + hf * 32 + c * 16, ul);
       }
       l += (sum[0].x + sum[0].y) + (sum[1].x + sum[1].y);
       tmem_st_wait();
@@ -398,6 +413,12 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_consta
     if (n > 0) {
       guard_wait(&o_full[w], 0, dead);
       tc_fence_after();
+      {                                                    // the row's sum
+        float* x = xch + w * 2 * PA_ROWS + r;
+        x[hf * PA_ROWS] = l;
+        asm volatile("bar.sync %0, 256;" ::"r"(3 + w) : "memory");
+        l += x[(hf ^ 1) * PA_ROWS];
+      }
       float f;
       if (p.sink) {
         const float sk = p.sink[live ? h : g * p.per] * PA_LOG2E, M = fmaxf(m, sk), c = pa_ex2(m - M);
@@ -413,7 +434,7 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_consta
       if (gt && p.gate_heads && live) f = f / (1.0f + expf(-__bfloat162float(gt[0])));
       const bool per_channel = gt != nullptr && !p.gate_heads;
 #pragma unroll 1
-      for (int c = 0; c < 4; ++c) {
+      for (int c = 2 * hf; c < 2 * hf + 2; ++c) {
         uint32_t u[32];
         tmem_ld_32x32b_x32(o_col + c * 32, u);
         tmem_ld_wait();
@@ -452,10 +473,10 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_consta
       }
     }
   }
-  if (threadIdx.x == 8 * 32 && *dead) guard_drain();
+  if (threadIdx.x == PA_SOFT * 32 && *dead) guard_drain();
   tc_fence_before();
   __syncthreads();
-  if (warp == 9) {
+  if (warp == PA_SOFT + 1) {
     tc_fence_after();
     tmem_dealloc(tmem, 512);
   }
@@ -503,7 +524,7 @@ int encode_rows(CUtensorMap* m, const void* ptr, int64_t cols, int64_t rows, int
 template <int NA, bool BIAS, typename QT>
 int launch_prompt_attn(const CUtensorMap& kmap, const CUtensorMap& rmap, const CUtensorMap& vmap, const PromptAttnParams& p,
                        int G, int n_seq, cudaStream_t st) {
-  const size_t smem = 1024 + PaCfg<NA>::TILES + PaCfg<NA>::BARS * 8 + 16 + (BIAS ? 16 * (size_t)p.per * p.tab_ld : 0);
+  const size_t smem = PaCfg<NA>::TILES + PaCfg<NA>::BARS * 8 + 16 + 4 * PA_ROWS * 4 + (BIAS ? 16 * (size_t)p.per * p.tab_ld : 0);
   B200_CHECK_ARG(smem <= 227 * 1024, "prompt_attn: %d query heads per key head do not fit in shared memory", p.per);
   auto kern = prompt_attn_kernel<NA, BIAS, QT>;
   B200_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
