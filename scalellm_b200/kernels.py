@@ -44,7 +44,8 @@ def _p(t: Optional[torch.Tensor]) -> Optional[int]:
 
 
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    """The current stream's handle (without the stream object: this runs on every call)."""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def _check_i32(*ts: torch.Tensor) -> None:
@@ -210,7 +211,7 @@ def dense_gemm(a: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tenso
     if a.stride(0) % 8 or a.data_ptr() % 16:
         a = a.contiguous()
     if out is None:
-        out = torch.empty((M, N), dtype=torch.bfloat16, device=a.device)
+        out = a.new_empty((M, N), dtype=torch.bfloat16)
     if M == 0:
         return out
     ws = _workspace("dense", a.device, int(_lib.load().b200_dense_workspace_bytes(M, N, K)))
@@ -505,8 +506,9 @@ def w4a16_gemm(a: torch.Tensor, packed: torch.Tensor, N: int, group_size: int,
     assert a.dim() == 2 and a.dtype == torch.bfloat16 and a.stride(1) == 1
     M, K = a.shape
     if out is None:
-        out = torch.empty((M, N), dtype=torch.bfloat16, device=a.device)
-    assert out.dtype == torch.bfloat16 and out.stride(1) == 1 and out.shape == (M, N)
+        out = a.new_empty((M, N))
+    else:
+        assert out.dtype == torch.bfloat16 and out.stride(1) == 1 and out.shape == (M, N)
     if workspace is None:
         workspace = w4a16_workspace(a.device, M, N, K)
     check(_lib.load().b200_w4a16_gemm(_p(out), _p(a), _p(packed), _p(bias), M, N, K, a.stride(0),

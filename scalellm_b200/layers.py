@@ -377,7 +377,7 @@ class _QLinearBase:
 
     def _gemm(self, x: torch.Tensor, bias: Optional[torch.Tensor]) -> torch.Tensor:
         self._ensure_packed()
-        x2 = x.reshape(-1, x.shape[-1])
+        x2 = x if x.dim() == 2 else x.reshape(-1, x.shape[-1])
         if self.perm is not None:
             x2 = kernels.permute_cols(x2, self.perm)
         if x2.shape[0] > _DENSE_PREFILL_ROWS and os.environ.get("B200_W4_PREFILL_DENSE", "1") != "0":
@@ -391,7 +391,7 @@ class _QLinearBase:
                 out = out + bias
             return out.view(*x.shape[:-1], self.N)
         out = kernels.w4a16_gemm(x2, self.packed, self.N, self.qa.group_size, bias=bias)
-        return out.view(*x.shape[:-1], self.N)
+        return out if x.dim() == 2 else out.view(*x.shape[:-1], self.N)
 
 
 def _shard_qtensors(sd: Dict[str, torch.Tensor], qa: QuantArgs, dim: int, rank: int, world: int,
@@ -512,6 +512,8 @@ def _dense_linear(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
     """F::linear of the reference's dense layers (parallel_linear.cpp:258,299): the tcgen05 stream
     kernel of csrc/dense.cu for bf16 on CUDA (B200_DENSE_IMPL=cublas: the library GEMM, for A/B)."""
     if os.environ.get("B200_DENSE_IMPL") != "cublas" and kernels.dense_supported(x, weight):
+        if x.dim() == 2:
+            return kernels.dense_gemm(x, weight)
         x2 = x.reshape(-1, x.shape[-1])
         return kernels.dense_gemm(x2, weight).view(*x.shape[:-1], weight.shape[0])
     return F.linear(x, weight)
