@@ -1,0 +1,43 @@
+"""GPU: the inputs of the gated delta rule made 16 rows a warp against the general kernel, which inputs that lie off
+the 4-value pieces take: portions around a row tile's and the filter's edges, carried and stale filter states, grouped
+heads.  Both compute in fp32 from the same inputs in another order: a filter is 4 products (8 roundings of 2^-24), a head's
+length a sum of 128 squares over the lanes (at most 16 in a row), so 2^-18 of the value covers either."""
+import pytest
+import torch
+
+from scalellm_b200 import kernels
+
+pytestmark = pytest.mark.gpu
+DEV, DIM, TAPS = "cuda", 128, 4
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("H,G", [(4, 2), (3, 3), (2, 1)])
+@pytest.mark.parametrize("lens", [[(8, 0)], [(15, 0), (16, 5), (17, 1)], [(1, 3), (2, 0), (3, 9), (40, 2)], [(33, 0), (130, 64)]])
+def test_tiles_of_rows_agree_with_the_general_kernel(lens, H, G, dtype):
+    g = torch.Generator(device=DEV).manual_seed(len(lens) * 10 + H)
+    rows, n_seq = sum(a for a, _ in lens), len(lens)
+    nqk, nv = G * DIM, H * DIM
+    rnd = lambda *s: torch.randn(s, generator=g, device=DEV)
+    width = 2 * nqk + nv + 4
+    src, dec = rnd(rows, width).to(dtype), rnd(rows, H * DIM).to(dtype)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    q_cu = i32([0] + list(torch.tensor([a for a, _ in lens]).cumsum(0)))
+    pos = i32([b + i for a, b in lens for i in range(a)])
+    seq = i32([s for s, (a, _) in enumerate(lens) for _ in range(a)])
+    slots = i32([n_seq - i for i in range(n_seq)])
+    par = [0.5 * rnd(n, TAPS) for n in (nqk, nqk, nv)] + [rnd(H), rnd(H * DIM)]
+    state = rnd(n_seq + 1, TAPS - 1, 2 * nqk + nv)
+    got = []
+    for shift in (0, 1):                       # a column off the pieces: the general kernel
+        buf = torch.zeros(rows, width + 4, dtype=dtype, device=DEV)
+        buf[:, shift: shift + width] = src
+        cut = lambda a, b: buf[:, shift + a: shift + b]
+        fs = state.clone()
+        got.append([*kernels.gated_delta_prepare(cut(0, nqk), cut(nqk, 2 * nqk), cut(2 * nqk, 2 * nqk + nv),
+                                                 cut(2 * nqk + nv, 2 * nqk + nv + H), dec, *par, fs, q_cu, pos, seq, slots, H,
+                                                 G, DIM, DIM, 1e-6), fs])
+    for name, a, b in zip(("q", "k", "v", "decay", "beta"), *got):
+        assert bool(torch.isfinite(a).all()), name
+        assert bool(((a - b).abs() <= 2.0 ** -18 * b.abs() + 2.0 ** -22).all()), (name, float((a - b).abs().max()))
+    assert torch.equal(got[0][5], got[1][5])   # inputs kept as they came

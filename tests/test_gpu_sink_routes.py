@@ -1,0 +1,41 @@
+"""GPU: prompt steps of the distance-bias attention over ordered keys against the kernel that walks the blocks, over the forms
+that the rule between them accepts: lengths on both sides of it, grouped heads, gates, window, values that are the keys,
+output columns of a wider matrix.  Both round the probabilities to bf16 before P V (2^-8 each) and the result once:
+|a - b| <= (2 x 2^-8 + 2 x 2^-8) max|v| of what is summed with weights of 1 or less."""
+import pytest
+import torch
+
+from scalellm_b200 import kernels
+
+pytestmark = pytest.mark.gpu
+DEV, D = "cuda", 128
+
+
+@pytest.mark.parametrize("lens", [[(64, 192)], [(63, 400), (1, 300)], [(300, 0), (17, 500)], [(130, 127), (5, 260), (257, 600)]])
+@pytest.mark.parametrize("per,bias,gate,window,same,pad", [(4, True, "channels", 0, False, 0), (1, False, "", 200, False, 8),
+                                                           (8, True, "heads", 0, True, 0), (2, True, "", 64, False, 0)])
+def test_both_routes_agree(lens, per, bias, gate, window, same, pad, monkeypatch):
+    g = torch.Generator(device=DEV).manual_seed(per + len(lens))
+    G, bs, n = 2, 16, len(lens)
+    H, rows = G * per, sum(a for a, _ in lens)
+    nb = [-(-(a + b) // bs) for a, b in lens]
+    rnd = lambda *s: torch.randn(s, generator=g, device=DEV)
+    kc = rnd((sum(nb) + 2) * bs, G, D).bfloat16()
+    vc = kc if same else rnd((sum(nb) + 2) * bs, G, D).bfloat16()
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    cu = lambda v: i32([0] + list(torch.tensor(v).cumsum(0)))
+    table = (torch.randperm(sum(nb), generator=torch.Generator().manual_seed(3)) * bs).to(torch.int32).to(DEV)
+    q = rnd(rows, H, D)
+    r1, r2 = (0.1 + 0.4 * torch.rand(2, H, generator=g, device=DEV)) if bias else (None, None)
+    sink = rnd(H)
+    gt = {"": None, "channels": rnd(rows, H * D).bfloat16(), "heads": rnd(rows, H).bfloat16()}[gate]
+    got = []
+    for impl in (None, "tc"):
+        monkeypatch.setenv("B200_SINK_ATTN_IMPL", impl) if impl else monkeypatch.delenv("B200_SINK_ATTN_IMPL", raising=False)
+        out = torch.zeros(rows, H * D + pad, dtype=torch.bfloat16, device=DEV)
+        kernels.sink_attn(q, kc, vc, r1, r2, sink, cu([a for a, _ in lens]), cu([a + b for a, b in lens]), table, cu(nb),
+                          i32([s for s, (a, _) in enumerate(lens) for _ in range(a)]), bs, D ** -0.5, n,
+                          max(a for a, _ in lens), max(a + b for a, b in lens), 0, gt, 1.0, out[:, : H * D], window)
+        got.append(out.double())
+    assert bool(torch.isfinite(got[0]).all()) and bool((got[0][:, H * D:] == 0).all())
+    assert float((got[0] - got[1]).abs().max()) <= 4 * 2.0 ** -8 * float(vc.float().abs().max())
