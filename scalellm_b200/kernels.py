@@ -1402,7 +1402,7 @@ SINK_ATTN_DECODE_TC_MIN_GROUP = 2
 # From how many query rows (tokens x query heads per key head) of the longest portion and how many keys a sequence, on
 # average, prompt steps run on csrc/prompt_attn.cu.  Below, a row tile is mostly padding, or the pass that orders the keys
 # is not made up for (16 heads, whole layer on the device: 4 x 128 tokens 46 us against 44 without it, 1 x 64 tokens over
-# 2 112 keys 95 against 170, 16 x 32 over 1 032 keys 74 against 107, 4 x 2 048 tokens 319 against 628).
+# 2 112 keys 98 against 170, 16 x 32 over 1 032 keys 70 against 107, 4 x 2 048 tokens 306 against 628).
 SINK_PROMPT_MIN_ROWS = 64
 SINK_PROMPT_MIN_KEYS = 256
 

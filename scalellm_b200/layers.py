@@ -753,7 +753,7 @@ class LatentAttention:
         """Whether this step makes keys and values of the latents (csrc/prompt_attn.cu) or attends in the latent space.
         The latter costs 2 (2 rank + rot_dim) FLOPs per (query, key) pair and head, the former 2 (dim + vdim + rot_dim) and
         a product over all keys of the step's sequences; the rates are what the kernels reach (16 heads, whole layer on the
-        device: 1 x 64 tokens over 2 112 keys 94 us against 134, 16 x 64 over 2 064 250 against 713, 1 x 300 over 4 300 157
+        device: 1 x 64 tokens over 2 112 keys 92 us against 134, 16 x 64 over 2 064 237 against 713, 1 x 300 over 4 300 155
         against 1 096; the 40 us are what 4 x 128 tokens, 107 us, do not make up for)."""
         if self.kv_proj is None or os.environ.get("B200_LATENT_IMPL") is not None or not kernels.prompt_attn_available():
             return False
